@@ -133,11 +133,18 @@ struct cansfz_ctx {
 
 namespace {
 
+// Zeroed device memory of the context.  The clearing runs on the context's
+// stream, as everything that writes the buffer afterwards does: the legacy
+// default stream does not order with a non-blocking one, so a clearing there
+// (behind a caller's own work) could land on top of what was written since.
 template <typename T>
 int dalloc(cansfz_ctx* c, T** p, size_t n) {
   void* q = nullptr;
   if (cudaMalloc(&q, n * sizeof(T) + 256) != cudaSuccess) return CANSFZ_ERR_NOMEM;
-  if (cudaMemset(q, 0, n * sizeof(T) + 256) != cudaSuccess) return CANSFZ_ERR_CUDA;
+  if (cudaMemsetAsync(q, 0, n * sizeof(T) + 256, c->st) != cudaSuccess) {
+    cudaFree(q);
+    return CANSFZ_ERR_CUDA;
+  }
   c->allocs.push_back(q);
   *p = (T*)q;
   return CANSFZ_OK;
@@ -433,7 +440,8 @@ int setup_solver(cansfz_ctx* c) {
   off_rz = host.size(); host.insert(host.end(), rz.begin(), rz.end());
   int rc = dalloc(c, &c->d_solver, host.size() + 2);
   if (rc) return rc;
-  CK(cudaMemcpy(c->d_solver, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice));
+  CK(cudaMemcpyAsync(c->d_solver, host.data(), host.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
+  CK(cudaStreamSynchronize(c->st));
   double* D = c->d_solver;
   c->pl.lam = D + off_lam;
   c->pl.a = D + off_a;
@@ -452,7 +460,8 @@ int setup_solver(cansfz_ctx* c) {
     float* F = nullptr;
     rc = dalloc(c, &F, hf.size() + 4);
     if (rc) return rc;
-    CK(cudaMemcpy(F, hf.data(), hf.size() * sizeof(float), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(F, hf.data(), hf.size() * sizeof(float), cudaMemcpyHostToDevice, c->st));
+    CK(cudaStreamSynchronize(c->st));
     for (int d = 0; d < 2; ++d) {
       lps[d]->twf = (const float2*)(F + off_tw[d]);
       lps[d]->tw2f = (const float2*)(F + off_tw2[d]);
@@ -807,7 +816,9 @@ int cansfz_create(const cansfz_params* prm, void* stream, cansfz_ctx** out) {
     for (auto* v : {&c->dzc, &c->dzf, &c->dzci, &c->dzfi, &c->gvr_c, &c->gvr_f, &c->zc, &c->zf})
       gh.insert(gh.end(), v->begin(), v->end());
     if ((rc = dalloc(c, &c->d_grid, gh.size()))) return fail(rc);
-    if (cudaMemcpy(c->d_grid, gh.data(), gh.size() * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess)
+    if (cudaMemcpyAsync(c->d_grid, gh.data(), gh.size() * sizeof(double), cudaMemcpyHostToDevice, c->st) !=
+            cudaSuccess ||
+        cudaStreamSynchronize(c->st) != cudaSuccess)
       return fail(CANSFZ_ERR_CUDA);
   }
   const int S = nz + 2;
@@ -1213,7 +1224,8 @@ int cansfz_ensemble_step(cansfz_ensemble* e, int nsteps, int* status_out) {
           }
         }
         CK(cudaMalloc(&e->argtab[par], total));
-        CK(cudaMemcpy(e->argtab[par], host.data(), total, cudaMemcpyHostToDevice));
+        CK(cudaMemcpyAsync(e->argtab[par], host.data(), total, cudaMemcpyHostToDevice, e->st));
+        CK(cudaStreamSynchronize(e->st));
       }
       cudaGraph_t graph;
       CK(cudaStreamBeginCapture(e->st, cudaStreamCaptureModeThreadLocal));
