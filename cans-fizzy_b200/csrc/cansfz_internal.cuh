@@ -189,12 +189,17 @@ struct PoissonPlan {
   double* zdf;
   float* zpivf;
   float* zdff;
+  // the same for column 0 alone (nz values), the singular mode's
+  double* zpiv0;
+  double* zdf0;
+  float* zpiv0f;
+  float* zdf0f;
   // the FP32 solve's x and y transforms as tensor-core GEMMs (k_xform_gemm.cu):
   // split-BF16 matrices [0] forward, [1] backward; null: the FFT kernels
   const uint16_t* gx[2];
   const uint16_t* gy[2];
-  // z solve of grids with many columns: 0 the partitioned tile solve where
-  // it applies, 1 one column per thread (cansfz_plan.zsolve)
+  // z solve: 0 the partitioned tile solve where it applies, 1 one column per
+  // thread (cansfz_plan.zsolve)
   int zmode;
   // x and y transforms of the periodic kind: 0 the two-pass register
   // kernels where the length allows, 1 the one-warp-per-line (x) and
@@ -375,8 +380,9 @@ int xform_gemm_set_attributes();
 void launch_xform_gemm(const Launch& L, const Geo& g, int mode, bool add, const uint16_t* bmat, int n,
                        const void* src, void* dst, double normfft, DevScalars* sc);
 // the z systems' elimination factors of `pl` (FP64, or FP32 for the mixed
-// form) into piv/df, evaluated exactly as the solve's forward sweep does
-void launch_z_factors(const Launch& L, const Geo& g, const PoissonPlan& pl, bool f32, void* piv, void* df);
+// form) of the first ncol columns into piv/df, evaluated exactly as the
+// solve's forward sweep does
+void launch_z_factors(const Launch& L, const Geo& g, const PoissonPlan& pl, bool f32, int ncol, void* piv, void* df);
 
 // z-marching tile kernels (k_tiles.cu), TI = double (drop-in) or float (mixed form)
 template <typename TI>

@@ -336,7 +336,13 @@ int alloc_f32_solver(cansfz_ctx* c) {
   if (c->pl.zper && !c->pl.work2f && (rc = dalloc(c, &c->pl.work2f, nint))) return rc;
   if (!c->pl.zpivf && zsolve_factored(c)) {
     if ((rc = dalloc(c, &c->pl.zpivf, nint)) || (rc = dalloc(c, &c->pl.zdff, nint))) return rc;
-    launch_z_factors(c->L, c->g, c->pl, true, c->pl.zpivf, c->pl.zdff);
+    launch_z_factors(c->L, c->g, c->pl, true, c->g.nx * c->g.ny, c->pl.zpivf, c->pl.zdff);
+    CK(cudaGetLastError());
+  }
+  if (!c->pl.zpiv0f && c->pl.zsing && z_part_ok(c->g, c->pl)) {
+    const size_t n = (size_t)c->n[2];
+    if ((rc = dalloc(c, &c->pl.zpiv0f, n)) || (rc = dalloc(c, &c->pl.zdf0f, n))) return rc;
+    launch_z_factors(c->L, c->g, c->pl, true, 1, c->pl.zpiv0f, c->pl.zdf0f);
     CK(cudaGetLastError());
   }
   return CANSFZ_OK;
@@ -484,7 +490,12 @@ int setup_solver(cansfz_ctx* c) {
   // them
   if (zsolve_factored(c)) {
     if ((rc = dalloc(c, &c->pl.zpiv, nint)) || (rc = dalloc(c, &c->pl.zdf, nint))) return rc;
-    launch_z_factors(c->L, c->g, c->pl, false, c->pl.zpiv, c->pl.zdf);
+    launch_z_factors(c->L, c->g, c->pl, false, nx * ny, c->pl.zpiv, c->pl.zdf);
+    CK(cudaGetLastError());
+  }
+  if (c->pl.zsing && z_part_ok(c->g, c->pl)) {
+    if ((rc = dalloc(c, &c->pl.zpiv0, (size_t)nz)) || (rc = dalloc(c, &c->pl.zdf0, (size_t)nz))) return rc;
+    launch_z_factors(c->L, c->g, c->pl, false, 1, c->pl.zpiv0, c->pl.zdf0);
     CK(cudaGetLastError());
   }
   if (P.form == CANSFZ_FORM_MIXED && P.refine_sweeps >= 0) {
@@ -2132,7 +2143,7 @@ int cansfz_autotune(cansfz_ctx* c, const char* cache_file, cansfz_plan* chosen, 
   try_knob(&cansfz_plan::momentum_slots, {24, 48, 96});
   try_knob(&cansfz_plan::tile_tma, {1, 0});
   if (c->wrap) try_knob(&cansfz_plan::ghost_images, {1, 0});
-  if (z_part_ok(c->g, c->pl) && !c->pl.zpiv) try_knob(&cansfz_plan::zsolve, {0, 1});
+  if (z_part_ok(c->g, c->pl)) try_knob(&cansfz_plan::zsolve, {0, 1});
   if (poisson_y2_applies(c->pl)) try_knob(&cansfz_plan::line_transforms, {0, 1});
   if (c->mixed && c->sweeps >= 0 && (xform_gemm_length(c->n[0]) || xform_gemm_length(c->n[1])))
     try_knob(&cansfz_plan::fp32_transforms, {0, 1});

@@ -1367,10 +1367,10 @@ __global__ void __launch_bounds__(128) k_zsolve(int ncol, int nz, const double* 
 
 // ---------------------------------------------------------------------------
 // z, partitioned: a tile of 32 columns with all nz levels in shared memory,
-// the levels split into P = 8 chunks of CH levels, one warp per chunk and one
-// lane per column.  The spectral buffer is read once and written once (the
-// column solve above reads and writes each level twice), and 256 threads
-// share each column's elimination instead of one.
+// the levels split into P chunks of at most CH levels, one warp per chunk and
+// one lane per column.  The spectral buffer is read once and written once (the
+// column solve above reads and writes each level twice), and P warps share
+// each column's elimination instead of one thread.
 //
 //   A  each chunk eliminates its interior rows s+1..e-1 twice with running
 //      scalars only: downwards with x_s as a parameter, which turns row e
@@ -1382,18 +1382,30 @@ __global__ void __launch_bounds__(128) k_zsolve(int ncol, int nz, const double* 
 //      (forward sweep into shared memory, the c/pivot factors in registers,
 //      back substitution).
 //
+// Chunk w holds nz/P levels, the first nz%P chunks one more (so any nz from
+// 3P to CH*P); EXACT: every chunk has CH levels.  What bounds it depends on
+// the grid: with many columns the FP64 reciprocals and the shared memory (two
+// blocks per SM at nz = 256), with few the length of the chain of dependent
+// steps, CH + 2P + 2P + 2CH against the column sweep's 2 nz (a whole step at 64x64x128: 203 -> 184 us, at 64x2x128: 138 -> 126 us, the solve itself 28 -> 9 us).
+//
 // The order of elimination differs from gaussel's (src/solver.f90:151-177)
 // only by round-off for these diagonally dominant systems (|b + lambda| >=
 // |a| + |c|).  The one singular system, the (0,0) mode of an all-periodic/
 // Neumann problem, whose eps-shifted pivot (src/solver.f90:163-167) fixes
-// the solution's constant, is solved by one thread of block 0 in gaussel's
-// own order (thomas_column's operations) from a copy of its right-hand
-// side, while the rest of the grid runs.
+// the solution's constant, is solved by one more block in gaussel's own
+// order (thomas_column's operations, the factors read where the plan has
+// them); the tile of column 0 leaves that column's result to it (what its
+// lane reads there meanwhile, right-hand side or solution, goes nowhere).
 // ---------------------------------------------------------------------------
 constexpr int ZP_NC = 32;  // columns per tile
-constexpr int ZP_P = 8;    // chunks (warps) per tile
-// the chunk lengths built (nz = 8 * CH)
+// the chunk lengths built (a chunk of fewer levels runs in the next longer one)
 #define CANSFZ_FOR_ZCHUNKS(X) X(8) X(12) X(16) X(24) X(32)
+// chunks of a column of nz levels: 8 up to 256 levels, 16 up to 512, none beyond or below 24
+__host__ __device__ constexpr int zpart_chunks(int nz) { return nz < 24 ? 0 : (nz <= 256 ? 8 : (nz <= 512 ? 16 : 0)); }
+__host__ __device__ constexpr int zpart_len(int nz) {
+  const int n = zpart_chunks(nz) ? (nz + zpart_chunks(nz) - 1) / zpart_chunks(nz) : 0;
+  return n <= 8 ? 8 : n <= 12 ? 12 : n <= 16 ? 16 : n <= 24 ? 24 : 32;
+}
 
 __device__ __forceinline__ void cp16_cg(void* sdst, const void* gsrc) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(sdst);
@@ -1401,37 +1413,94 @@ __device__ __forceinline__ void cp16_cg(void* sdst, const void* gsrc) {
 }
 
 template <typename T>
-constexpr size_t zpart_smem(int nz) {
-  return sizeof(T) * ((size_t)nz * ZP_NC + (size_t)8 * ZP_P * ZP_NC + (size_t)2 * ZP_P * ZP_NC + 2 * (size_t)nz);
+constexpr size_t zpart_smem(int nz, int P) {
+  return sizeof(T) * ((size_t)nz * ZP_NC + (size_t)8 * P * ZP_NC + (size_t)2 * P * ZP_NC);
 }
 
-template <typename T, int CH>
+// the singular column: gaussel's elimination order and rounding, by one thread
+// (its operands staged in shared memory by the block)
+template <typename T>
+__device__ void zsolve_serial0(int ncol, int nz, const double* __restrict__ a, const double* __restrict__ b,
+                               const double* __restrict__ c, const T* __restrict__ piv0, const T* __restrict__ df0,
+                               T* __restrict__ work, int zsing, T* __restrict__ sm) {
+  typedef Rn<T> R;
+  T* pv = sm;
+  T* dd = sm + nz;
+  T* zz = sm + 2 * nz;
+  T* aa = sm + 3 * nz;
+  const bool have = piv0 != nullptr && df0 != nullptr;
+  for (int l = threadIdx.x; l < nz; l += blockDim.x) {
+    pv[l] = work[(size_t)l * ncol];
+    aa[l] = (T)__ldg(a + l);
+    if (have) {
+      zz[l] = __ldg(piv0 + l);
+      dd[l] = __ldg(df0 + l);
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const bool pin = sizeof(T) == 4 && zsing;
+    T dprev = 0, pprev = 0;
+    if (have) {
+#pragma unroll 8
+      for (int l = 0; l < nz; ++l) {
+        const T z = zz[l];
+        pprev = l == 0 ? R::mul(pv[l], z) : R::mul(R::sub(pv[l], R::mul(aa[l], pprev)), z);
+        pv[l] = pprev;
+      }
+    } else {
+      for (int l = 0; l < nz; ++l) {
+        const T z = piv_inv<T>(l, nz, (T)__ldg(b + l), (T)0, aa[l], dprev, pin);
+        dprev = R::mul((T)__ldg(c + l), z);
+        dd[l] = dprev;
+        pprev = l == 0 ? R::mul(pv[l], z) : R::mul(R::sub(pv[l], R::mul(aa[l], pprev)), z);
+        pv[l] = pprev;
+      }
+    }
+    T pnext = pv[nz - 1];
+#pragma unroll 8
+    for (int l = nz - 2; l >= 0; --l) {
+      pnext = R::sub(pv[l], R::mul(dd[l], pnext));
+      pv[l] = pnext;
+    }
+  }
+  __syncthreads();
+  for (int l = threadIdx.x; l < nz; l += blockDim.x) work[(size_t)l * ncol] = pv[l];
+}
+
+template <typename T, int CH, int P, bool EXACT>
 struct ZSolvePart {
   static __device__ __forceinline__ void run(const Blk& bk, int ncol, int nz, const double* __restrict__ lam,
       const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
-      const DevScalars* __restrict__ sc, T* __restrict__ work, int zsing) {
-    typedef Rn<T> R;
+      const T* __restrict__ piv0, const T* __restrict__ df0, const DevScalars* __restrict__ sc,
+      T* __restrict__ work, int zsing) {
     if (HALTED(sc)) return;
     static_assert(CH >= 3, "a chunk needs an interior row");
-    constexpr int NC = ZP_NC, P = ZP_P;
+    constexpr int NC = ZP_NC;
     extern __shared__ __align__(16) unsigned char smraw[];
     T* tile = reinterpret_cast<T*>(smraw);        // [nz][NC]
     T* red = tile + (size_t)nz * NC;               // [2P][4][NC]: sub, diag, sup, rhs of the reduced rows
     T* xb = red + (size_t)8 * P * NC;              // [2P][NC]: x_s, x_e of every chunk
-    T* s0 = xb + (size_t)2 * P * NC;               // [2][nz]: column 0 of block 0 (serial path)
-    const int col0 = bk.x * NC;
+    const bool serial0 = zsing && __ldg(lam) == 0.;
+    if (bk.x == bk.nx - 1) {  // the extra block
+      if (serial0) zsolve_serial0<T>(ncol, nz, a, b, c, piv0, df0, work, zsing, tile);
+      return;
+    }
+    const int col0 = bk.x * NC, cols = EXACT ? NC : min(NC, ncol - col0);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int s = w * CH, e = s + CH - 1;
-    // each warp stages its own chunk's rows (16-byte copies of rows of NC
+    const int base = EXACT ? CH : nz / P, rem = EXACT ? 0 : nz % P;
+    const int len = EXACT ? CH : base + (w < rem ? 1 : 0);
+    const int s = EXACT ? w * CH : w * base + min(w, rem), e = s + len - 1;
+    const bool in = EXACT || lane < cols;
+    // each warp stages its own chunk's rows (16-byte copies of rows of
     // consecutive columns) and starts on them without waiting for the others
     constexpr int PER = 16 / (int)sizeof(T), CPR = NC / PER;
-    for (int q = lane; q < CH * CPR; q += 32) {
+    for (int q = lane; q < len * CPR; q += 32) {
       const int l = s + q / CPR, cc = (q % CPR) * PER;
-      cp16_cg(tile + (size_t)l * NC + cc, work + (size_t)l * ncol + col0 + cc);
+      if (EXACT || cc < cols) cp16_cg(tile + (size_t)l * NC + cc, work + (size_t)l * ncol + col0 + cc);
     }
     asm volatile("cp.async.commit_group;\n" ::);
-    const T lm = (T)__ldg(lam + col0 + lane);
-    const bool serial0 = col0 == 0 && __ldg(lam) == 0.;
+    const T lm = (T)__ldg(lam + (in ? col0 + lane : 0));
     asm volatile("cp.async.wait_group 0;\n" ::);
     __syncwarp();
     // ---- A: the chunk's two reduced rows.  The downward sweep's pivot
@@ -1442,6 +1511,7 @@ struct ZSolvePart {
       T D = 0, Y = 0, F = 0, U = 0, Z = 0, G = 0;
 #pragma unroll
       for (int t = 0; t < CH - 2; ++t) {
+        if (!EXACT && t >= len - 2) break;  // the same for the whole warp
         const int id = s + 1 + t, iu = e - 1 - t;
         const T ad = (T)__ldg(a + id), cd = (T)__ldg(c + id), bd = (T)__ldg(b + id) + lm;
         const T au = (T)__ldg(a + iu), cu = (T)__ldg(c + iu), bu = (T)__ldg(b + iu) + lm;
@@ -1468,8 +1538,6 @@ struct ZSolvePart {
       Re[1 * NC + lane] = be - ae * D;
       Re[2 * NC + lane] = w == P - 1 ? (T)0 : ce;
       Re[3 * NC + lane] = tile[e * NC + lane] - ae * Y;
-      if (serial0 && lane == 0)
-        for (int l = s; l <= e; ++l) s0[l] = tile[(size_t)l * NC];  // column 0's right-hand side
     }
     __syncthreads();
     // ---- B: the reduced system of the 2P chunk-end values
@@ -1494,22 +1562,23 @@ struct ZSolvePart {
     }
     __syncthreads();
     // ---- C: the chunk's interior rows with x_s and x_e known, then its rows
-    // out (column 0 of block 0 waits for the serial solve)
+    // out (column 0 of a singular problem is the extra block's)
     {
       const T xs = xb[(2 * w) * NC + lane], xe = xb[(2 * w + 1) * NC + lane];
       T Y = 0;
 #pragma unroll
       for (int t = 0; t < CH - 2; ++t) {
+        if (!EXACT && t >= len - 2) break;
         const int i = s + 1 + t;
         const T ai = (T)__ldg(a + i), ci = (T)__ldg(c + i);
         T rhs = tile[i * NC + lane];
         if (t == 0) rhs -= ai * xs;
-        if (t == CH - 3) rhs -= ci * xe;  // row e-1: x_e is known, no super-diagonal left
+        if (t == (EXACT ? CH : len) - 3) rhs -= ci * xe;  // row e-1: x_e is known, no super-diagonal left
         Y = (t == 0 ? rhs : rhs - ai * Y) * rp[t];
         tile[i * NC + lane] = Y;
       }
       T* out = work + col0 + lane;
-      const bool keep = !(serial0 && lane == 0);
+      const bool keep = in && !(serial0 && col0 + lane == 0);
       if (keep) {
         out[(size_t)s * ncol] = xs;
         out[(size_t)e * ncol] = xe;
@@ -1518,40 +1587,20 @@ struct ZSolvePart {
       T x = Y;
 #pragma unroll
       for (int t = CH - 4; t >= 0; --t) {
+        if (!EXACT && t > len - 4) continue;
         const int i = s + 1 + t;
         x = tile[i * NC + lane] - ((T)__ldg(c + i) * rp[t]) * x;
         if (keep) out[(size_t)i * ncol] = x;
       }
     }
-    if (serial0 && threadIdx.x == 0) {
-      // gaussel's elimination order and rounding for the singular mode
-      T* pv = s0;
-      T* dd = s0 + nz;
-      const bool pin = sizeof(T) == 4 && zsing;
-      T dprev = 0, pprev = 0;
-      for (int l = 0; l < nz; ++l) {
-        const T z = piv_inv<T>(l, nz, (T)__ldg(b + l), (T)0, (T)__ldg(a + l), dprev, pin);
-        const T d = R::mul((T)__ldg(c + l), z);
-        const T pn = l == 0 ? R::mul(pv[l], z) : R::mul(R::sub(pv[l], R::mul((T)__ldg(a + l), pprev)), z);
-        dd[l] = d;
-        pv[l] = pn;
-        dprev = d;
-        pprev = pn;
-      }
-      T pnext = 0;
-      for (int l = nz - 1; l >= 0; --l) {
-        if (l < nz - 1) pv[l] = R::sub(pv[l], R::mul(dd[l], pnext));
-        pnext = pv[l];
-        work[(size_t)l * ncol] = pv[l];
-      }
-    }
   }
 };
-template <typename T, int CH>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) k_zsolve_part(int ncol, int nz, const double* __restrict__ lam,
-    const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
+template <typename T, int CH, int P, bool EXACT>
+__global__ void __launch_bounds__(32 * P, P == 8 ? (sizeof(T) == 4 ? 4 : 2) : 1) k_zsolve_part(int ncol, int nz,
+    const double* __restrict__ lam, const double* __restrict__ a, const double* __restrict__ b,
+    const double* __restrict__ c, const T* __restrict__ piv0, const T* __restrict__ df0,
     const DevScalars* __restrict__ sc, T* __restrict__ work, int zsing) {
-  ZSolvePart<T, CH>::run(blk_here(), ncol, nz, lam, a, b, c, sc, work, zsing);
+  ZSolvePart<T, CH, P, EXACT>::run(blk_here(), ncol, nz, lam, a, b, c, piv0, df0, sc, work, zsing);
 }
 
 // periodic z: gaussel_periodic (src/solver.f90:107-149)
@@ -1692,19 +1741,26 @@ static void set_attr_len() {
 }
 
 // opt the transform kernels into > 48 KB of dynamic shared memory (once)
-template <typename T, int CH>
+template <typename T, int CH, int P, bool EXACT>
 static void set_attr_zpart() {
-  cudaFuncSetAttribute(k_zsolve_part<T, CH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)zpart_smem<T>(CH * ZP_P));
+  cudaFuncSetAttribute(k_zsolve_part<T, CH, P, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)zpart_smem<T>(CH * P, P));
   // all of the unified L1/shared storage as shared memory: 2 FP64 or 4 FP32
-  // tiles per SM
-  cudaFuncSetAttribute(k_zsolve_part<T, CH>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  // tiles per SM at 256 levels
+  cudaFuncSetAttribute(k_zsolve_part<T, CH, P, EXACT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+}
+template <typename T>
+static void set_attrs_zpart() {
+#define X(C) set_attr_zpart<T, C, 8, true>(); set_attr_zpart<T, C, 8, false>();
+  CANSFZ_FOR_ZCHUNKS(X)
+#undef X
+  set_attr_zpart<T, 24, 16, true>(); set_attr_zpart<T, 24, 16, false>();
+  set_attr_zpart<T, 32, 16, true>(); set_attr_zpart<T, 32, 16, false>();
 }
 
 void poisson_set_attributes() {
-#define X(C) set_attr_zpart<double, C>(); set_attr_zpart<float, C>();
-  CANSFZ_FOR_ZCHUNKS(X)
-#undef X
+  set_attrs_zpart<double>();
+  set_attrs_zpart<float>();
   set_attr_len<double, 0>();
   set_attr_len<float, 0>();
 #define X(M) set_attr_len<double, M>(); set_attr_len<float, M>();
@@ -1820,8 +1876,8 @@ template <typename T> static const T* zdf(const PoissonPlan& pl);
 template <> const double* zdf<double>(const PoissonPlan& pl) { return pl.zdf; }
 template <> const float* zdf<float>(const PoissonPlan& pl) { return pl.zdff; }
 
-void launch_z_factors(const Launch& L, const Geo& g, const PoissonPlan& pl, bool f32, void* piv, void* df) {
-  const int ncol = g.nx * g.ny, tb = 128;
+void launch_z_factors(const Launch& L, const Geo& g, const PoissonPlan& pl, bool f32, int ncol, void* piv, void* df) {
+  const int tb = 128;
   if (f32)
     k_z_factors<float><<<(ncol + tb - 1) / tb, tb, 0, L.st>>>(ncol, g.nz, pl.lam, pl.a, pl.b, pl.c, pl.zsing,
                                                              static_cast<float*>(piv), static_cast<float*>(df));
@@ -1830,38 +1886,51 @@ void launch_z_factors(const Launch& L, const Geo& g, const PoissonPlan& pl, bool
                                                               static_cast<double*>(piv), static_cast<double*>(df));
 }
 
-template <typename T, int CH>
-static void z_part_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl, const DevScalars* sc) {
+template <typename T> static const T* zpiv0(const PoissonPlan& pl);
+template <> const double* zpiv0<double>(const PoissonPlan& pl) { return pl.zpiv0; }
+template <> const float* zpiv0<float>(const PoissonPlan& pl) { return pl.zpiv0f; }
+template <typename T> static const T* zdf0(const PoissonPlan& pl);
+template <> const double* zdf0<double>(const PoissonPlan& pl) { return pl.zdf0; }
+template <> const float* zdf0<float>(const PoissonPlan& pl) { return pl.zdf0f; }
+
+template <typename T, int CH, int P, bool EXACT>
+static void z_part_go(const Launch& Lc, const Geo& g, const PoissonPlan& pl, const DevScalars* sc) {
   const int ncol = g.nx * g.ny;
-  kgo<ZSolvePart<T, CH>, 256, sizeof(T) == 4 ? 4 : 2>(Lc, k_zsolve_part<T, CH>, ncol / ZP_NC, 32 * ZP_P, zpart_smem<T>(g.nz), ncol,
-                                 g.nz, pl.lam, pl.a, pl.b, pl.c, sc, wbuf<T>(pl), pl.zsing);
+  constexpr int MINB = P == 8 ? (sizeof(T) == 4 ? 4 : 2) : 1;
+  // the tiles of columns, and the block of the singular column
+  kgo<ZSolvePart<T, CH, P, EXACT>, 32 * P, MINB>(Lc, k_zsolve_part<T, CH, P, EXACT>, (ncol + ZP_NC - 1) / ZP_NC + 1,
+                                                 32 * P, zpart_smem<T>(g.nz, P), ncol, g.nz, pl.lam, pl.a, pl.b, pl.c,
+                                                 zpiv0<T>(pl), zdf0<T>(pl), sc, wbuf<T>(pl), pl.zsing);
+}
+template <typename T, int CH, int P>
+static void z_part_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl, const DevScalars* sc) {
+  if (g.nz == CH * P && (g.nx * g.ny) % ZP_NC == 0) z_part_go<T, CH, P, true>(Lc, g, pl, sc);
+  else z_part_go<T, CH, P, false>(Lc, g, pl, sc);
 }
 
 bool poisson_y2_applies(const PoissonPlan& pl) {
   return (pl.py.kind == 0 && y2_length(pl.py.m)) || (pl.px.kind == 0 && y2_length(pl.px.m));
 }
 
-// the partitioned solve serves non-periodic z with nz = 8 * CH and whole
-// tiles of columns; few-column grids keep the factored solve
+// the partitioned solve serves non-periodic z of 24 to 512 levels; the columns
+// of a tile are copied in 16-byte pieces (two FP64 or four FP32 columns)
 bool z_part_ok(const Geo& g, const PoissonPlan& pl) {
-  const int ncol = g.nx * g.ny;
-  if (pl.zper || ncol % ZP_NC != 0 || g.nz % ZP_P != 0) return false;
-  switch (g.nz / ZP_P) {
-#define X(C) case C:
-    CANSFZ_FOR_ZCHUNKS(X)
-#undef X
-    return true;
-    default: return false;
-  }
+  return !pl.zper && (g.nx * g.ny) % 4 == 0 && zpart_chunks(g.nz) != 0;
 }
 
 template <typename T>
 static void z_pass(const Launch& Lc, const Geo& g, const PoissonPlan& pl, const DevScalars* sc) {
   const int ncol = g.nx * g.ny;
   const int tb = 64;
-  if (pl.zmode != 1 && !(zpiv<T>(pl) && zdf<T>(pl)) && z_part_ok(g, pl)) {
-    switch (g.nz / ZP_P) {
-#define X(C) case C: z_part_len<T, C>(Lc, g, pl, sc); return;
+  if (pl.zmode != 1 && z_part_ok(g, pl)) {
+    const int len = zpart_len(g.nz);
+    if (zpart_chunks(g.nz) == 16) {
+      if (len == 24) z_part_len<T, 24, 16>(Lc, g, pl, sc);
+      else z_part_len<T, 32, 16>(Lc, g, pl, sc);
+      return;
+    }
+    switch (len) {
+#define X(C) case C: z_part_len<T, C, 8>(Lc, g, pl, sc); return;
       CANSFZ_FOR_ZCHUNKS(X)
 #undef X
       default: break;

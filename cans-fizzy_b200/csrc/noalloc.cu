@@ -146,6 +146,7 @@ extern "C" int cansfz_solver_static(const int n[3], const char cbc[3][2], double
   pl.c = c;
   pl.normfft = normfft;
   pl.zper = 0;
+  pl.zsing = (cbc[2][0] != 'D' && cbc[2][1] != 'D') ? 1 : 0;
   pl.work = s.scratch;
 
   cansfz::Geo g{};

@@ -332,10 +332,9 @@ typedef struct cansfz_plan {
   int32_t phase_slots;      /* blocks per SM that the z split of the ACDI/THINC
                                and Youngs tiles aims at (default 24)          */
   int32_t momentum_slots;   /* the same for the momentum tile (default 48)   */
-  int32_t zsolve;           /* Poisson z solve of grids with >= 32768 columns:
-                               0 the partitioned 32-column tiles where nz is
-                               8 x (8, 12, 16, 24 or 32), 1 one column per
-                               thread                                         */
+  int32_t zsolve;           /* Poisson z solve: 0 the partitioned 32-column
+                               tiles where z is not periodic and has 24 to
+                               512 levels, 1 one column per thread            */
   int32_t fp32_transforms;  /* mixed form's FP32 solve: 0 tensor-core GEMMs
                                where the line lengths allow, 1 FFTs           */
   double  ms_per_step;      /* step time measured with the plan by
