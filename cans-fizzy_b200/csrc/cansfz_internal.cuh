@@ -374,7 +374,7 @@ double xform_coef(int kind, int dir, int n, int j, int k);
 std::vector<uint16_t> xform_bmat(int kind, int dir, int n);
 bool xform_gemm_length(int n);
 bool z_part_ok(const Geo& g, const PoissonPlan& pl);
-// the x or y transforms have a two-pass register kernel (periodic kind, 64-256 points)
+// the x or y transforms have a two-pass register kernel (periodic kind, 64-512 points)
 bool poisson_y2_applies(const PoissonPlan& pl);
 int xform_gemm_set_attributes();
 void launch_xform_gemm(const Launch& L, const Geo& g, int mode, bool add, const uint16_t* bmat, int n,

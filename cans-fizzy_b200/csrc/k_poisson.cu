@@ -1121,6 +1121,244 @@ __global__ void __launch_bounds__(FftY2<T, DIR, MC>::NT, 3) k_fft_y2(Geo g, Line
 }
 
 // ---------------------------------------------------------------------------
+// Lines of 512 points (m = 256 = 16 x 16) in the same two register passes,
+// but with one column k1 per thread in the pair pass: two columns of 16 points
+// would need twice the registers.  Z_{m-k} of column k1 is column 16 - k1's,
+// which a lane of the same warp holds (the y kernel assigns the columns so;
+// the 16 threads of an x line are half a warp), so the pairing is a shuffle
+// (columns 0 and 8 pair with themselves).  256 threads hold 16 lines: rows of
+// 16 consecutive x positions, 128 bytes, in y.  64 KiB of shared memory (x: 68
+// KiB, with a k1 pitch of 17) and 128 registers allow two blocks per SM.
+// Against the shared-memory Stockham kernels, four radix stages with a block
+// barrier each: a step at 512x512x256 9.66 -> 8.78 ms, at 512x256x256 (x lines only) 4.60 -> 4.40 ms.
+// ---------------------------------------------------------------------------
+constexpr int kW = 16;  // both DFT lengths, and lines per CTA
+template <typename T>
+constexpr size_t w512_smem(bool x) { return sizeof(cx<T>) * kW * kW * (x ? kW + 1 : kW); }
+
+template <typename T, int DIR>
+struct FftYW {
+  static constexpr int NT = kW * kW;
+  static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
+      const DevScalars* __restrict__ sc, T* __restrict__ work) {
+    if (HALTED(sc)) return;
+    constexpr int M = kW * kW;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    cx<T>* sb = reinterpret_cast<cx<T>*>(smraw);  // [k1][j2][line]
+    const int nx = g.nx;
+    const int l = threadIdx.x % kW, q = threadIdx.x / kW;
+    const int i = bk.x * kW + l;
+    const bool in = i < nx;
+    T* col = work + (size_t)bk.y * nx * (2 * M) + (in ? i : 0);
+    auto row = [&](int r) -> T& { return col[(size_t)r * nx]; };
+    // the pair pass: warp wq holds columns wq and 16 - wq (0 and 8)
+    const int wq = threadIdx.x >> 5, hf = (threadIdx.x >> 4) & 1;
+    const int k1 = wq == 0 ? 8 * hf : (hf ? kW - wq : wq);
+    if (DIR > 0) {
+      {
+        cx<T> z[kW], y[kW];
+#pragma unroll
+        for (int j1 = 0; j1 < kW; ++j1) {
+          const int r = 2 * (q + kW * j1);
+          z[j1] = in ? mk<T>(row(r), row(r + 1)) : mk<T>(0, 0);
+        }
+        RegDft<T, kW, -1, 1>::run(z, y);
+#pragma unroll
+        for (int a = 0; a < kW; ++a) sb[(a * kW + q) * kW + l] = (a > 0) ? cmul<T>(y[a], TW<T>(pl, q * a)) : y[a];
+      }
+      __syncthreads();
+      cx<T> a[kW], z[kW];
+#pragma unroll
+      for (int j2 = 0; j2 < kW; ++j2) a[j2] = sb[(k1 * kW + j2) * kW + l];
+      RegDft<T, kW, -1, 1>::run(a, z);
+#pragma unroll
+      for (int k2 = 0; k2 < kW; ++k2) {
+        cx<T> zm;
+        if (wq > 0) zm = shfl_xor_c<T>(z[kW - 1 - k2], 16);
+        else zm = hf ? z[kW - 1 - k2] : z[(kW - k2) % kW];
+        const int k = k1 + kW * k2;
+        const cx<T> X = real_fwd_Xc<T>(pl, z[k2], zm, k);
+        if (in) {
+          if (k == 0) {  // packed: r_0, r_m
+            row(0) = X.x;
+            row(1) = real_fwd_Xc<T>(pl, z[0], z[0], M).x;
+          } else {
+            row(2 * k) = X.x;
+            row(2 * k + 1) = X.y;
+          }
+        }
+      }
+    } else {
+      {
+        cx<T> x[kW], z[kW];
+#pragma unroll
+        for (int k2 = 0; k2 < kW; ++k2) {
+          const int k = k1 + kW * k2;
+          x[k2] = in ? mk<T>(row(2 * k), row(2 * k + 1)) : mk<T>(0, 0);
+        }
+        const bool first = k1 == 0;  // slot 0 holds X_0 and X_m, both real
+        const T xm = x[0].y;
+        if (first) x[0].y = (T)0;
+#pragma unroll
+        for (int k2 = 0; k2 < kW; ++k2) {
+          cx<T> xmk;
+          if (wq > 0) xmk = shfl_xor_c<T>(x[kW - 1 - k2], 16);
+          else xmk = hf ? x[kW - 1 - k2] : (k2 == 0 ? mk<T>(xm, (T)0) : x[(kW - k2) % kW]);
+          z[k2] = real_bwd_Z<T>(pl, x[k2], xmk, k1 + kW * k2);
+        }
+        RegDft<T, kW, +1, 1>::run(z, x);
+#pragma unroll
+        for (int j2 = 0; j2 < kW; ++j2)
+          sb[(k1 * kW + j2) * kW + l] = j2 > 0 ? cmul<T>(x[j2], cconj<T>(TW<T>(pl, j2 * k1))) : x[j2];
+      }
+      __syncthreads();
+      cx<T> u[kW], z[kW];
+#pragma unroll
+      for (int a = 0; a < kW; ++a) u[a] = sb[(a * kW + q) * kW + l];
+      RegDft<T, kW, +1, 1>::run(u, z);
+      if (in) {
+#pragma unroll
+        for (int j1 = 0; j1 < kW; ++j1) {
+          const int r = 2 * (q + kW * j1);
+          row(r) = z[j1].x;
+          row(r + 1) = z[j1].y;
+        }
+      }
+    }
+  }
+};
+template <typename T, int DIR>
+__global__ void __launch_bounds__(FftYW<T, DIR>::NT, 2) k_fft_y512(Geo g, LinePlan pl,
+                                                                  const DevScalars* __restrict__ sc,
+                                                                  T* __restrict__ work) {
+  FftYW<T, DIR>::run(blk_here(), g, pl, sc, work);
+}
+
+// x lines of 512 points: the forward transform of a halo field's interior (or,
+// FUSED, of fillps's right-hand side), and the backward one into a halo field
+template <typename T, bool FUSED>
+struct FftXWFwd {
+  static constexpr int NT = kW * kW, P = kW + 1;
+  static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
+      const DevScalars* __restrict__ sc, const double* __restrict__ src, const double* __restrict__ u,
+      const double* __restrict__ v, const double* __restrict__ w, const Phys& ph, T* __restrict__ work) {
+    if (HALTED(sc)) return;
+    constexpr int M = kW * kW, N = 2 * M;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int q = threadIdx.x % kW, l = threadIdx.x / kW, lane = threadIdx.x & 31;
+    cx<T>* sl = reinterpret_cast<cx<T>*>(smraw) + l * (kW * P);  // [line][k1][j2]
+    const int gl = bk.x * kW + l;
+    const bool in = gl < g.ny * g.nz;
+    const int jj = in ? gl % g.ny + 1 : 1, kk = in ? gl / g.ny + 1 : 1;
+    const int cb = g.h(1, jj, kk);
+    const double dti = FUSED ? sc->dti : 0.;
+    const double dtidxi = dti * g.dxi, dtidyi = dti * g.dyi, dzk = FUSED ? dti * g.dzfi[kk] : 0.;
+    auto get = [&](int c) -> double {
+      if (FUSED)
+        return ph.rho0 * ((__ldg(w + c) - __ldg(w + c - g.sxy)) * dzk + (__ldg(v + c) - __ldg(v + c - g.sx)) * dtidyi +
+                          (__ldg(u + c) - __ldg(u + c - 1)) * dtidxi);
+      return __ldg(src + c);
+    };
+    {
+      cx<T> z[kW], y[kW];
+#pragma unroll
+      for (int j1 = 0; j1 < kW; ++j1) {
+        const int c = cb + 2 * (q + kW * j1);
+        z[j1] = in ? mk<T>((T)get(c), (T)get(c + 1)) : mk<T>(0, 0);
+      }
+      RegDft<T, kW, -1, 1>::run(z, y);
+#pragma unroll
+      for (int a = 0; a < kW; ++a) sl[a * P + q] = (a > 0) ? cmul<T>(y[a], TW<T>(pl, q * a)) : y[a];
+    }
+    __syncwarp();  // a line's 16 threads are half a warp
+    cx<T> a[kW], z[kW];
+#pragma unroll
+    for (int j2 = 0; j2 < kW; ++j2) a[j2] = sl[q * P + j2];
+    RegDft<T, kW, -1, 1>::run(a, z);
+    cx<T>* out = reinterpret_cast<cx<T>*>(work + (size_t)(in ? gl : 0) * N);
+    const int src_lane = (lane & 16) | ((kW - q) & (kW - 1));
+#pragma unroll
+    for (int k2 = 0; k2 < kW; ++k2) {
+      cx<T> zm = shfl_c<T>(z[kW - 1 - k2], src_lane);
+      if (q == 0) zm = z[(kW - k2) % kW];
+      const int k = q + kW * k2;
+      cx<T> X = real_fwd_Xc<T>(pl, z[k2], zm, k);
+      if (k2 == 0 && q == 0) X.y = real_fwd_Xc<T>(pl, z[0], z[0], M).x;  // packed: r_0, r_m
+      if (in) out[k] = X;
+    }
+  }
+};
+template <typename T, bool FUSED>
+__global__ void __launch_bounds__(256, 2) k_fft_x512_fwd(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
+    const double* __restrict__ src, const double* __restrict__ u, const double* __restrict__ v,
+    const double* __restrict__ w, Phys ph, T* __restrict__ work) {
+  FftXWFwd<T, FUSED>::run(blk_here(), g, pl, sc, src, u, v, w, ph, work);
+}
+
+template <typename T, bool ADD>
+struct FftXWBwd {
+  static constexpr int NT = kW * kW, P = kW + 1;
+  static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
+      const DevScalars* __restrict__ sc, const T* __restrict__ work, double normfft, double* __restrict__ dst,
+      int wrap) {
+    if (HALTED(sc)) return;
+    constexpr int N = 2 * kW * kW;
+    extern __shared__ __align__(16) unsigned char smraw[];
+    const int q = threadIdx.x % kW, l = threadIdx.x / kW, lane = threadIdx.x & 31;
+    cx<T>* sl = reinterpret_cast<cx<T>*>(smraw) + l * (kW * P);
+    const int gl = bk.x * kW + l;
+    const bool in = gl < g.ny * g.nz;
+    {
+      const cx<T>* row = reinterpret_cast<const cx<T>*>(work + (size_t)(in ? gl : 0) * N);
+      cx<T> x[kW], z[kW];
+#pragma unroll
+      for (int k2 = 0; k2 < kW; ++k2) x[k2] = row[q + kW * k2];
+      const T xm = x[0].y;  // slot 0 holds X_0 and X_m, both real
+      if (q == 0) x[0].y = (T)0;
+      const int src_lane = (lane & 16) | ((kW - q) & (kW - 1));
+#pragma unroll
+      for (int k2 = 0; k2 < kW; ++k2) {
+        cx<T> xmk = shfl_c<T>(x[kW - 1 - k2], src_lane);
+        if (q == 0) xmk = k2 == 0 ? mk<T>(xm, (T)0) : x[(kW - k2) % kW];
+        z[k2] = real_bwd_Z<T>(pl, x[k2], xmk, q + kW * k2);
+      }
+      RegDft<T, kW, +1, 1>::run(z, x);
+#pragma unroll
+      for (int j2 = 0; j2 < kW; ++j2) sl[q * P + j2] = j2 > 0 ? cmul<T>(x[j2], cconj<T>(TW<T>(pl, j2 * q))) : x[j2];
+    }
+    __syncwarp();  // a line's 16 threads are half a warp
+    cx<T> uu[kW], z[kW];
+#pragma unroll
+    for (int a = 0; a < kW; ++a) uu[a] = sl[a * P + q];
+    RegDft<T, kW, +1, 1>::run(uu, z);
+    if (!in) return;
+    const int jj = gl % g.ny + 1, kk = gl / g.ny + 1;
+    const int cb = g.h(1, jj, kk);
+    const int oy = ADD ? 0 : wrap_oy(g, wrap, jj), oz = ADD ? 0 : wrap_oz(g, wrap, kk);
+#pragma unroll
+    for (int j1 = 0; j1 < kW; ++j1) {
+      const int j = q + kW * j1;
+      const int c = cb + 2 * j;  // x_{2j} at i = 2j + 1, x_{2j+1} at i = 2j + 2
+      if (ADD) {
+        dst[c] = dst[c] + (double)z[j1].x * normfft;
+        dst[c + 1] = dst[c + 1] + (double)z[j1].y * normfft;
+      } else {
+        const double o0 = (double)z[j1].x * normfft, o1 = (double)z[j1].y * normfft;
+        dst[c] = o0;
+        dst[c + 1] = o1;
+        store_images(c, wrap_ox(g, wrap, 2 * j + 1), oy, oz, [&](int h) { dst[h] = o0; });
+        store_images(c + 1, wrap_ox(g, wrap, 2 * j + 2), oy, oz, [&](int h) { dst[h] = o1; });
+      }
+    }
+  }
+};
+template <typename T, bool ADD>
+__global__ void __launch_bounds__(256, 2) k_fft_x512_bwd(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
+    const T* __restrict__ work, double normfft, double* __restrict__ dst, int wrap) {
+  FftXWBwd<T, ADD>::run(blk_here(), g, pl, sc, work, normfft, dst, wrap);
+}
+
+// ---------------------------------------------------------------------------
 // z: batched Thomas (dgtsv_homebrewed with the eps pivot shift, src/solver.f90:
 // 151-177 / src/solver_gpu.f90:179-203).  One column per thread; the forward
 // sweep writes p' in place and keeps d only at chunk ends (shared memory);
@@ -1758,7 +1996,22 @@ static void set_attrs_zpart() {
   set_attr_zpart<T, 32, 16, true>(); set_attr_zpart<T, 32, 16, false>();
 }
 
+template <typename T>
+static void set_attrs_w512() {
+  auto set = [](auto k, bool x) {
+    cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)w512_smem<T>(x));
+  };
+  set(k_fft_y512<T, 1>, false);
+  set(k_fft_y512<T, -1>, false);
+  set(k_fft_x512_fwd<T, true>, true);
+  set(k_fft_x512_fwd<T, false>, true);
+  set(k_fft_x512_bwd<T, true>, true);
+  set(k_fft_x512_bwd<T, false>, true);
+}
+
 void poisson_set_attributes() {
+  set_attrs_w512<double>();
+  set_attrs_w512<float>();
   set_attrs_zpart<double>();
   set_attrs_zpart<float>();
   set_attr_len<double, 0>();
@@ -1798,6 +2051,18 @@ static void x_forward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl,
       else
         kgo<FftX2Fwd<T, false, MC>, X::NT, 3>(Lc, k_fft_x2_fwd<T, false, MC>, g2, X::NT, 0, g, pl.px, sc, src,
                                              nullptr, nullptr, nullptr, pz, wbuf<T>(pl));
+      return;
+    }
+  }
+  if constexpr (MC == 256) {
+    if (pl.px.kind == 0 && pl.lmode == 0) {
+      const dim3 g5((nlines + kW - 1) / kW);
+      if (fused)
+        kgo<FftXWFwd<T, true>, 256, 2>(Lc, k_fft_x512_fwd<T, true>, g5, 256, w512_smem<T>(true), g, pl.px, sc, nullptr,
+                                       u, v, w, *ph, wbuf<T>(pl));
+      else
+        kgo<FftXWFwd<T, false>, 256, 2>(Lc, k_fft_x512_fwd<T, false>, g5, 256, w512_smem<T>(true), g, pl.px, sc, src,
+                                        nullptr, nullptr, nullptr, pz, wbuf<T>(pl));
       return;
     }
   }
@@ -1845,6 +2110,16 @@ static void y_pass_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl, co
         kgo<FftY2<T, 1, MC>, Y::NT, 3>(Lc, k_fft_y2<T, 1, MC>, g2, Y::NT, 0, g, pl.py, sc, wbuf<T>(pl));
       else
         kgo<FftY2<T, -1, MC>, Y::NT, 3>(Lc, k_fft_y2<T, -1, MC>, g2, Y::NT, 0, g, pl.py, sc, wbuf<T>(pl));
+      return;
+    }
+  }
+  if constexpr (MC == 256) {
+    if (pl.py.kind == 0 && pl.lmode == 0) {
+      const dim3 g5((g.nx + kW - 1) / kW, g.nz);
+      if (dir > 0)
+        kgo<FftYW<T, 1>, 256, 2>(Lc, k_fft_y512<T, 1>, g5, 256, w512_smem<T>(false), g, pl.py, sc, wbuf<T>(pl));
+      else
+        kgo<FftYW<T, -1>, 256, 2>(Lc, k_fft_y512<T, -1>, g5, 256, w512_smem<T>(false), g, pl.py, sc, wbuf<T>(pl));
       return;
     }
   }
@@ -1909,7 +2184,8 @@ static void z_part_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl, co
 }
 
 bool poisson_y2_applies(const PoissonPlan& pl) {
-  return (pl.py.kind == 0 && y2_length(pl.py.m)) || (pl.px.kind == 0 && y2_length(pl.px.m));
+  auto two_pass = [](const LinePlan& p) { return p.kind == 0 && (y2_length(p.m) || p.m == kW * kW); };
+  return two_pass(pl.px) || two_pass(pl.py);
 }
 
 // the partitioned solve serves non-periodic z of 24 to 512 levels; the columns
@@ -1967,6 +2243,13 @@ static void x_backward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl
       using X = FftX2Bwd<T, ADD, MC>;
       kgo<FftX2Bwd<T, ADD, MC>, X::NT, 4>(Lc, k_fft_x2_bwd<T, ADD, MC>, (nlines + X::L - 1) / X::L, X::NT, 0, g,
                                          pl.px, sc, wbuf<T>(pl), pl.normfft, dst, ADD ? 0 : Lc.wrap);
+      return;
+    }
+  }
+  if constexpr (MC == 256) {
+    if (pl.px.kind == 0 && pl.lmode == 0) {
+      kgo<FftXWBwd<T, ADD>, 256, 2>(Lc, k_fft_x512_bwd<T, ADD>, (nlines + kW - 1) / kW, 256, w512_smem<T>(true), g,
+                                    pl.px, sc, wbuf<T>(pl), pl.normfft, dst, ADD ? 0 : Lc.wrap);
       return;
     }
   }

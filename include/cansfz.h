@@ -349,7 +349,7 @@ typedef struct cansfz_plan {
                                skip those copies (default); 0 the fills copy
                                them.  The ghost values are the same bits     */
   int32_t line_transforms;  /* x and y transforms of the periodic kind with
-                               64, 128 or 256 points: 0 two register passes
+                               64 to 512 = 2^n points: 0 two register passes
                                per line with one block barrier (default), 1
                                one warp per line (x lines of 128 or 256) or
                                the shared-memory Stockham FFT                */
