@@ -551,7 +551,7 @@ static void momentum_go(const Launch& L, const Geo& g, const Phys& ph, const Dev
                         const double* s, const SurfSplit& sp, TI* duo, TI* dvo, TI* dwo, double* uo, double* vo,
                         double* wo) {
   using S = tile::Shape<TYV>;
-  const int kz = tile::kz_of<TYV>(g, L.batched, L.nsm, L.mom_slots > 0 ? L.mom_slots : kMomSlots);
+  const int kz = tile::kz_of<TYV>(g, L.batched, L.nsm, L.mom_slots > 0 ? L.mom_slots : kMomSlots, TYV == 4 ? 4 : 5);
   // the staged fields' tensor maps: all eleven in the FP64 drop-in; the
   // seven FP64 ones (u v w psi, psio p po: entries 0-3 and 7-9) in the mixed
   // form, whose FP32 planes are element copies

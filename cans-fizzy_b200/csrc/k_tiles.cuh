@@ -58,9 +58,10 @@ inline dim3 grid_of(const Geo& g, int kz) {
 inline int rows_of(const Geo& g) { return g.ny <= 2 ? 2 : 8; }
 
 // z levels per block; `slots`: blocks per SM that the split aims at (the
-// ACDI and Youngs tiles 24, the momentum tile 48, measured at 256^3)
+// ACDI and Youngs tiles 24, the momentum tile 48, measured at 256^3), `res`:
+// blocks that are resident on an SM at a time
 template <int TYV>
-inline int kz_of(const Geo& g, int batched, int nsm, int slots = 24) {
+inline int kz_of(const Geo& g, int batched, int nsm, int slots, int res) {
   using S = Shape<TYV>;
   // in an ensemble the other cases keep the GPU busy: 32 levels per block
   // spend 6% on the two extra planes each block loads (25% at 8 levels)
@@ -68,10 +69,17 @@ inline int kz_of(const Geo& g, int batched, int nsm, int slots = 24) {
   // several waves of resident blocks on each of the device's SMs (148 on a
   // B200), so the last partial wave costs little; at least 8 levels per
   // block (each block loads two planes and evaluates one face/vertex plane
-  // beyond its own levels)
+  // beyond its own levels) -- unless so few blocks leave part of the device
+  // idle: then as few levels as make one wave, since a block's levels run one
+  // after the other and their latency is the kernel's time (8 levels
+  // against this rule: a step at 64x2x128 126 -> 97 us, 64x64x128 184 -> 176 us,
+  // 90x50x70 251 -> 235 us)
   const long long xy = (long long)((g.nx + S::TX - 1) / S::TX) * ((g.ny + S::TY - 1) / S::TY);
-  long long kz = (xy * g.nz) / ((long long)(nsm > 0 ? nsm : 148) * slots);
-  if (kz < 8) kz = 8;
+  const long long sm = nsm > 0 ? nsm : 148, levels = xy * g.nz;
+  long long lo = (levels + sm * res - 1) / (sm * res);
+  if (lo > 8) lo = 8;
+  long long kz = levels / (sm * slots);
+  if (kz < lo) kz = lo;
   if (kz > 64) kz = 64;
   return (int)kz;
 }
