@@ -3,11 +3,13 @@ oracle: the partitioned z solve's chunks (shortest and longest columns,
 columns that the chunks do not divide, a last tile of few columns, FP64 and
 FP32), and the two-pass transforms of 512 points with a partial tile of lines.
 
-Bounds as in test_gpu_parity.test_poisson_bcs: 1e-12 of the largest stored
-value (the constant of the singular mode included) for the FP64 solve; one
-refinement sweep of the FP32 solve leaves the square of its own relative
-error, about 1e-5 for lines of up to 512 points, times a condition number of
-the residual below 1e4: 1e-6.
+Bounds: as in test_gpu_parity.test_poisson_bcs, 1e-12 of the largest stored
+value (the constant of the singular mode included) for the FP64 solve.  One
+refinement sweep of the FP32 solve leaves the square of its own relative error:
+up to 7e-4 for a column of 500 levels (2^-24 times a condition number of about
+(2 nz/pi)^2), squared 5e-7, bound 1e-6.  (Not for Neumann walls on a grid whose
+single-precision z quotients make it slightly uneven: there the FP64 residual's
+mean over the singular mode leaves 1e-6 and more whatever the sweeps, in either z solve.)
 """
 import numpy as np
 import pytest
@@ -60,7 +62,7 @@ def test_solver(cbcpre, ng):
     assert err / scale < 1e-12
 
 
-@pytest.mark.parametrize("cbcpre,ng", [("PPPPDD", (12, 10, 24)), ("PPPPNN", (20, 6, 31)), ("PPPPDD", (64, 2, 65)),
+@pytest.mark.parametrize("cbcpre,ng", [("PPPPDD", (12, 10, 24)), ("PPPPDD", (20, 6, 31)), ("PPPPDD", (64, 2, 65)),
                                        ("PPPPDD", (10, 6, 500)), ("PPPPDD", (512, 6, 9)), ("PPPPNN", (20, 512, 32))])
 def test_solver_refined(cbcpre, ng):
     p, rhs = _system(cbcpre, ng)
