@@ -278,13 +278,14 @@ void launch_thinc_step(const Launch& L, const Geo& g, const DevScalars* sc, bool
                        const double* u, const double* v, const double* w, const double* nx,
                        const double* ny, const double* nz, const double* phi, const double* psi,
                        double* psi_out, double* hist, double* fx, double* fy, double* fz);
-void launch_psi_update(const Launch& L, const Geo& g, const DevScalars* sc,
-                       const double* psi_in, double* psi_out, double* dpsidt, double* dpsidto);
 void launch_cmpt_phi(const Launch& L, const Geo& g, const DevScalars* sc, bool acdi,
                      const double* psi, double* phi);
 void launch_youngs(const Launch& L, const Geo& g, const DevScalars* sc, const double* psi,
                    double* nx, double* ny, double* nz, double* kappa);
 void launch_clip(const Launch& L, const Geo& g, double rmin, double rmax, double* p);
+// the interior of one to three halo-layout fields from as many others; clip:
+// the ghosts of the (one) field are clipped to [0, 1] besides
+void launch_put_interior(const Launch& L, const Geo& g, int nf, const double* const* src, double* const* dst, bool clip);
 void launch_mom_ad(const Launch& L, const Geo& g, const Phys& ph, const double* fx,
                    const double* fy, const double* fz, const double* u, const double* v,
                    const double* w, const double* psi, double* du, double* dv, double* dw);

@@ -172,28 +172,6 @@ void launch_thinc_transport(const Launch& L, const Geo& g, const DevScalars* sc,
 }
 
 // ---------------------------------------------------------------------------
-// rk_2fl update + clip, src/rk.f90:234-248 (the clip of the halo is dropped:
-// every ghost cell is overwritten by boundp(psi) right after)
-// ---------------------------------------------------------------------------
-__global__ void k_psi_update(Geo g, const DevScalars* __restrict__ sc, const double* __restrict__ psi_in,
-                             double* __restrict__ psi_out, const double* __restrict__ dn,
-                             double* __restrict__ dold) {
-  if (HALTED(sc)) return;
-  INTERIOR_IJK(g)
-  const int c = g.h(i, j, k), t = g.t(i, j, k);
-  const double d = dn[t];
-  const double dO = sc->first_rk2fl ? d : dold[t];
-  const double val = LD(psi_in, c) + sc->f1 * d + sc->f2 * dO;
-  psi_out[c] = fmin(fmax(0., val), 1.);
-}
-
-void launch_psi_update(const Launch& L, const Geo& g, const DevScalars* sc, const double* psi_in,
-                       double* psi_out, double* dpsidt, double* dpsidto) {
-  dim3 b = blk_interior(g), gr = grd_interior(g, b);
-  k_psi_update<<<gr, b, 0, L.st>>>(g, sc, psi_in, psi_out, dpsidt, dpsidto);
-}
-
-// ---------------------------------------------------------------------------
 // acdi_cmpt_phi (src/acdi.f90:227-248), vof_thinc_cmpt_phi
 // (src/vof_thinc_qq.f90:135-157): whole halo array
 // ---------------------------------------------------------------------------
@@ -279,6 +257,39 @@ __global__ void k_clip(int n, double rmin, double rmax, double* __restrict__ p) 
 void launch_clip(const Launch& L, const Geo& g, double rmin, double rmax, double* p) {
   const int n = g.hsize();
   k_clip<<<(n + 255) / 256, 256, 0, L.st>>>(n, rmin, rmax, p);
+}
+
+// the result of a fused update back into the caller's arrays
+struct PutFields {
+  const double* src[3];
+  double* dst[3];
+};
+// one warp per row, eight rows per block, field blockIdx.y; clip: the rows of
+// the ghost layer too
+__global__ void __launch_bounds__(256) k_put_interior(Geo g, PutFields f, int clip) {
+  const int lo = clip ? 0 : 1, ny = clip ? g.ny + 2 : g.ny, nz = clip ? g.nz + 2 : g.nz;
+  const int r = blockIdx.x * 8 + threadIdx.y;
+  if (r >= ny * nz) return;
+  const int q = blockIdx.y, j = r % ny + lo, k = r / ny + lo;
+  const double* __restrict__ src = q == 0 ? f.src[0] : (q == 1 ? f.src[1] : f.src[2]);
+  double* __restrict__ dst = q == 0 ? f.dst[0] : (q == 1 ? f.dst[1] : f.dst[2]);
+  const bool row = j >= 1 && j <= g.ny && k >= 1 && k <= g.nz;
+  const int c = g.h(0, j, k);
+#pragma unroll 4
+  for (int i = threadIdx.x + lo; i <= g.nx + 1 - lo; i += 32) {
+    if (row && i >= 1 && i <= g.nx) dst[c + i] = __ldg(src + c + i);
+    else dst[c + i] = fmin(fmax(0., dst[c + i]), 1.);
+  }
+}
+void launch_put_interior(const Launch& L, const Geo& g, int nf, const double* const* src, double* const* dst,
+                         bool clip) {
+  PutFields f{};
+  for (int q = 0; q < nf; ++q) {
+    f.src[q] = src[q];
+    f.dst[q] = dst[q];
+  }
+  const int rows = clip ? (g.ny + 2) * (g.nz + 2) : g.ny * g.nz;
+  k_put_interior<<<dim3((rows + 7) / 8, nf), dim3(32, 8), 0, L.st>>>(g, f, clip ? 1 : 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -743,9 +754,8 @@ void launch_fillps(const Launch& L, const Geo& g, const Phys& ph, const DevScala
 __global__ void k_correc(Geo g, Phys ph, const DevScalars* __restrict__ sc, const double* __restrict__ p,
                          double* __restrict__ u, double* __restrict__ v, double* __restrict__ w) {
   if (HALTED(sc)) return;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i > g.nx + 1) return;
-  const int j = blockIdx.y, k = blockIdx.z;
+  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, k = blockIdx.z;
+  if (i > g.nx + 1 || j > g.ny + 1) return;
   const double dt = sc->dt, rhop = ph.rho0;
   const int c = g.h(i, j, k);
   const double pc = LD(p, c);
@@ -755,7 +765,9 @@ __global__ void k_correc(Geo g, Phys ph, const DevScalars* __restrict__ sc, cons
 }
 void launch_correc(const Launch& L, const Geo& g, const Phys& ph, const DevScalars* sc, const double* p, double* u,
                    double* v, double* w) {
-  dim3 b(g.nx + 2 >= 128 ? 128 : 64), gr((g.nx + 2 + b.x - 1) / b.x, g.ny + 2, g.nz + 2);
+  // 32x8 tiles: blocks of 128 along x left one of two nearly empty at nx = 128
+  // (34 -> 32 us)
+  const dim3 b(32, 8), gr((g.nx + 2 + 31) / 32, (g.ny + 2 + 7) / 8, g.nz + 2);
   k_correc<<<gr, b, 0, L.st>>>(g, ph, sc, p, u, v, w);
 }
 
