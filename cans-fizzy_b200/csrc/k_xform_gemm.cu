@@ -20,8 +20,8 @@
 // Kernel structure (two persistent CTAs of 8 warps per SM, 128 lines per tile):
 //   * the tile's 128 lines x n samples stream through shared memory in chunks
 //     of 64 samples, one stage per CTA: while one CTA's chunk is on the
-//     tensor cores the other CTA of the SM loads and splits its next one.  Each thread loads 32 samples of one
-//     line (the next chunk's load is in flight while the tensor cores work on
+//     tensor cores the other CTA of the SM loads and splits its next one.  Each thread loads 32 samples
+//     (the next chunk's load is in flight while the tensor cores work on
 //     the current one), splits them and stores them in the canonical K-major
 //     layout of the MMA (8-row x 16-byte core matrices, no swizzle);
 //   * the matching 64-column chunk of F (hi and lo, precomputed on the host
@@ -54,6 +54,9 @@ constexpr int GM = 128;   // lines per tile (MMA M)
 constexpr int GKC = 64;   // samples per K chunk
 constexpr int GST = 1;    // stages per CTA (two CTAs share an SM and alternate)
 constexpr int GTHREADS = 256;
+// A's core matrices: 144 bytes from one to the next along K, so that the eight
+// that a warp's 4-byte stores of one line reach lie on different banks
+constexpr uint32_t GLBO = 144, GSBO = (GKC / 8) * GLBO;
 
 __device__ __forceinline__ uint32_t su32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -143,6 +146,18 @@ __device__ __forceinline__ void split_store(unsigned char* ahi, unsigned char* a
   *reinterpret_cast<uint4*>(alo + off) = make_uint4(l[0], l[1], l[2], l[3]);
 }
 
+// the same of two consecutive samples (4 bytes each)
+template <typename V>
+__device__ __forceinline__ void split_store2(unsigned char* ahi, unsigned char* alo, uint32_t off, V a, V b) {
+  const __nv_bfloat16 h0 = __float2bfloat16_rn((float)a), h1 = __float2bfloat16_rn((float)b);
+  const __nv_bfloat16 l0 = __float2bfloat16_rn((float)(a - (V)__bfloat162float(h0)));
+  const __nv_bfloat16 l1 = __float2bfloat16_rn((float)(b - (V)__bfloat162float(h1)));
+  *reinterpret_cast<uint32_t*>(ahi + off) =
+      (uint32_t)__bfloat16_as_ushort(h0) | ((uint32_t)__bfloat16_as_ushort(h1) << 16);
+  *reinterpret_cast<uint32_t*>(alo + off) =
+      (uint32_t)__bfloat16_as_ushort(l0) | ((uint32_t)__bfloat16_as_ushort(l1) << 16);
+}
+
 }  // namespace
 
 // MODE 0: x forward, lines (j,k) of an FP64 halo field -> FP32 spectral rows
@@ -159,30 +174,42 @@ struct GemmXform {
   double normfft;
 };
 
-// the 32 samples (four core rows) of one line that a thread stages per chunk
+// the 32 samples that a thread stages per chunk: in y half of one line's (four
+// core rows; a warp's lanes are consecutive x positions), in x, whose lines are
+// contiguous, two consecutive ones of each of the warp's 16 lines, so that a
+// warp reads 64 consecutive samples at a time (one line per thread read 32
+// rows at once, a sector each: x forward 87 -> 77 us, x backward 90 -> 75
+// us at 256^3)
 template <int MODE>
 struct LineVals {
   using T = typename std::conditional<MODE == 0, double, float>::type;
   T v[32];
 };
 
+// y: `base` and `live` of the thread's own line, samples from k0 on
+__device__ __forceinline__ void load_y(const GemmXform& p, bool live, size_t base, int k0, LineVals<1>& x) {
+  const float* sp = static_cast<const float*>(p.src) + base + (size_t)k0 * p.g.nx;
+#pragma unroll
+  for (int q = 0; q < 32; ++q) x.v[q] = live ? sp[(size_t)q * p.g.nx] : 0.f;
+}
+// x: lane i (i < 16) holds the start of the warp's line i, -1 past the last
 template <int MODE>
-__device__ __forceinline__ void load_line(const GemmXform& p, bool live, size_t base, int l, int k0,
-                                          LineVals<MODE>& x) {
-  if (MODE == 0) {
-    const double* sp = static_cast<const double*>(p.src) + base + k0;
+__device__ __forceinline__ void load_x(const GemmXform& p, int lbase, int k0, LineVals<MODE>& x) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll
-    for (int q = 0; q < 32; ++q) x.v[q] = live ? __ldg(sp + q) : 0.;
-  } else if (MODE == 1) {
-    const float* sp = static_cast<const float*>(p.src) + base + (size_t)k0 * p.g.nx;
-#pragma unroll
-    for (int q = 0; q < 32; ++q) x.v[q] = live ? sp[(size_t)q * p.g.nx] : 0.f;
-  } else {
-    const float4* sp = reinterpret_cast<const float4*>(static_cast<const float*>(p.src) + (size_t)l * p.n + k0);
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const float4 f = live ? sp[q] : make_float4(0.f, 0.f, 0.f, 0.f);
-      x.v[4 * q] = f.x; x.v[4 * q + 1] = f.y; x.v[4 * q + 2] = f.z; x.v[4 * q + 3] = f.w;
+  for (int i = 0; i < 16; ++i) {
+    const int b = __shfl_sync(0xffffffffu, lbase, i);
+    x.v[2 * i] = x.v[2 * i + 1] = 0;
+    if (b >= 0) {
+      if (MODE == 0) {
+        const double* sp = static_cast<const double*>(p.src) + b + k0 + 2 * lane;
+        x.v[2 * i] = __ldg(sp);
+        x.v[2 * i + 1] = __ldg(sp + 1);
+      } else {
+        const float2 f = *reinterpret_cast<const float2*>(static_cast<const float*>(p.src) + b + k0 + 2 * lane);
+        x.v[2 * i] = f.x;
+        x.v[2 * i + 1] = f.y;
+      }
     }
   }
 }
@@ -192,7 +219,7 @@ __global__ void __launch_bounds__(GTHREADS, 2) k_xform_gemm(GemmXform p, DevScal
   if (sc != nullptr && sc->halted) return;
   extern __shared__ __align__(1024) unsigned char smem[];
   const int n = p.n, nkc = n / GKC;
-  const uint32_t a_bytes = GM * GKC * 2, b_bytes = (uint32_t)n * GKC * 2;
+  const uint32_t a_bytes = GM / 8 * GSBO, b_bytes = (uint32_t)n * GKC * 2;
   const uint32_t stage_bytes = 2 * a_bytes + 2 * b_bytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + GST * stage_bytes);  // full[2], done[2], acc, fin
   uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 8);
@@ -221,28 +248,44 @@ __global__ void __launch_bounds__(GTHREADS, 2) k_xform_gemm(GemmXform p, DevScal
   int used[2] = {0, 0}, inflight[2] = {0, 0};
   bool fail = false, issued = false;
   int gch = 0;
-  // thread t stages half h = t / 128 (32 samples) of line r = t % 128 of the tile
+  const int lane = tid & 31;
+  // y: thread t stages half h = t / 128 (32 samples) of line r = t % 128 of the tile
   const int r = tid & (GM - 1), hh = tid / GM;
-  const uint32_t arow = (uint32_t)((r >> 3) * (GKC / 8)) * 128 + (uint32_t)(r & 7) * 16 + (uint32_t)hh * 4 * 128;
+  const uint32_t arow = (uint32_t)(r >> 3) * GSBO + (uint32_t)(r & 7) * 16 + (uint32_t)hh * 4 * GLBO;
+  // x: lane l stages samples 2l and 2l + 1 of the warp's 16 lines
+  const uint32_t apair = (uint32_t)(warp * 2) * GSBO + (uint32_t)(lane >> 2) * GLBO + (uint32_t)(lane & 3) * 4;
   // the epilogue: warp w reads TMEM lanes 32*(w%4).. (its lines), columns of half w/4
   const int er = (warp & 3) * 32 + (tid & 31), ecol0 = (warp >> 2) * (n / 2);
-  auto line_of = [&](int tile, int rr, bool& live, size_t& base) {
-    const int l = tile * GM + rr;
-    live = l < p.nlines;
-    if (MODE == 0 || MODE == 2) {
-      const int j = live ? l % p.g.ny : 0, k = live ? l / p.g.ny : 0;
-      base = (size_t)p.g.h(1, j + 1, k + 1);
-    } else {
-      const int x = live ? l % p.g.nx : 0, z = live ? l / p.g.nx : 0;
-      base = (size_t)z * p.g.nx * p.g.ny + x;
-    }
-    return l;
+  // where line l starts: in the spectral rows (x), between them (y), in the
+  // halo field (HALO); -1 past the last line
+  auto spec_base = [&](int l) -> int { return l < p.nlines ? l * n : -1; };
+  auto halo_base = [&](int l) -> int {
+    return l < p.nlines ? p.g.h(1, l % p.g.ny + 1, l / p.g.ny + 1) : -1;
+  };
+  auto y_base = [&](int l) -> size_t {
+    return l < p.nlines ? (size_t)(l / p.g.nx) * p.g.nx * p.g.ny + l % p.g.nx : 0;
   };
   LineVals<MODE> x;
-  bool live;
-  size_t base;
-  int l = line_of(blockIdx.x, r, live, base);
-  if (blockIdx.x < p.ntiles) load_line<MODE>(p, live, base, l, hh * 32, x);  // first chunk in flight
+  bool live = false;
+  size_t base = 0;
+  int lbase = -1;
+  auto next_tile = [&](int t) {
+    if (MODE == 1) {
+      live = t * GM + r < p.nlines;
+      base = y_base(t * GM + r);
+    } else {
+      const int l = t * GM + warp * 16 + (lane & 15);
+      lbase = MODE == 0 ? halo_base(l) : spec_base(l);
+    }
+  };
+  auto load = [&](int k0) {
+    if constexpr (MODE == 1) load_y(p, live, base, k0 + hh * 32, x);
+    else load_x<MODE>(p, lbase, k0, x);
+  };
+  if (blockIdx.x < p.ntiles) {
+    next_tile(blockIdx.x);
+    load(0);  // first chunk in flight
+  }
 
   for (int tile = blockIdx.x; tile < p.ntiles; tile += gridDim.x) {
     for (int kc = 0; kc < nkc; ++kc, ++gch) {
@@ -265,12 +308,18 @@ __global__ void __launch_bounds__(GTHREADS, 2) k_xform_gemm(GemmXform p, DevScal
         bulk_g2s(su32(blo), bsrc + b_bytes, b_bytes, bfull[s]);
         inflight[s] = 1;
       }
+      if (MODE == 1) {
 #pragma unroll
-      for (int g = 0; g < 4; ++g) {
-        typename LineVals<MODE>::T v8[8];
+        for (int g = 0; g < 4; ++g) {
+          typename LineVals<MODE>::T v8[8];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v8[q] = x.v[8 * g + q];
-        split_store(ahi, alo, arow + (uint32_t)g * 128, v8);
+          for (int q = 0; q < 8; ++q) v8[q] = x.v[8 * g + q];
+          split_store(ahi, alo, arow + (uint32_t)g * GLBO, v8);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i)
+          split_store2(ahi, alo, apair + (uint32_t)(i >> 3) * GSBO + (uint32_t)(i & 7) * 16, x.v[2 * i], x.v[2 * i + 1]);
       }
       fence_async_smem();
       __syncthreads();
@@ -280,8 +329,8 @@ __global__ void __launch_bounds__(GTHREADS, 2) k_xform_gemm(GemmXform p, DevScal
         const bool last = kc == nkc - 1;
         const int nt = last ? tile + (int)gridDim.x : tile;
         if (nt < p.ntiles) {
-          if (last) l = line_of(nt, r, live, base);
-          load_line<MODE>(p, live, base, l, (last ? 0 : (kc + 1) * GKC) + hh * 32, x);
+          if (last) next_tile(nt);
+          load(last ? 0 : (kc + 1) * GKC);
         }
       }
       if (tid == 0) {
@@ -293,8 +342,8 @@ __global__ void __launch_bounds__(GTHREADS, 2) k_xform_gemm(GemmXform p, DevScal
           tc_after();
 #pragma unroll
           for (int kk = 0; kk < GKC / 16; ++kk) {
-            const uint32_t ko = (uint32_t)kk * 2 * 128;
-            const uint64_t dah = sdesc(su32(ahi) + ko, lbo, sbo), dal = sdesc(su32(alo) + ko, lbo, sbo);
+            const uint32_t ko = (uint32_t)kk * 2 * 128, ka = (uint32_t)kk * 2 * GLBO;
+            const uint64_t dah = sdesc(su32(ahi) + ka, GLBO, GSBO), dal = sdesc(su32(alo) + ka, GLBO, GSBO);
             const uint64_t dbh = sdesc(su32(bhi) + ko, lbo, sbo), dbl = sdesc(su32(blo) + ko, lbo, sbo);
             mma_bf16(tmem, dah, dbh, idesc, (kc | kk) != 0 ? 1u : 0u);
             mma_bf16(tmem, dah, dbl, idesc, 1u);
@@ -312,45 +361,51 @@ __global__ void __launch_bounds__(GTHREADS, 2) k_xform_gemm(GemmXform p, DevScal
     if (__syncthreads_or(fail)) goto cleanup;
     tc_after();
     {
-      bool elive;
-      size_t ebase;
-      const int el = line_of(tile, er, elive, ebase);
       // x passes: a line's outputs are contiguous, so each warp turns its
       // 32 lines x 32 columns around in shared memory (the stages are idle
-      // now) and writes line by line, 32 consecutive columns per store
+      // now) and writes line by line, 32 consecutive columns per store; lane
+      // i holds the start of line i, and eight lines' old values (ADD) load
+      // together (one after the other: 189 -> 108 us at 256^3)
       float* tb = reinterpret_cast<float*>(smem) + warp * (32 * 33);
-      const int lane = tid & 31;
+      const int el = tile * GM + er;
+      const int eb = MODE == 1 ? 0 : (MODE == 0 ? spec_base(el) : halo_base(el));
+      const size_t yb = MODE == 1 ? y_base(el) : 0;
       for (int c0 = ecol0; c0 < ecol0 + n / 2; c0 += 32) {
         uint32_t v[32];
         tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0, v);
         if (MODE == 1) {
-          if (!elive) continue;
-          float* dp = static_cast<float*>(p.dst) + ebase + (size_t)c0 * p.g.nx;
+          if (el >= p.nlines) continue;
+          float* dp = static_cast<float*>(p.dst) + yb + (size_t)c0 * p.g.nx;
 #pragma unroll
           for (int q = 0; q < 32; ++q) dp[(size_t)q * p.g.nx] = __uint_as_float(v[q]);
         } else {
 #pragma unroll
           for (int q = 0; q < 32; ++q) tb[lane * 33 + q] = __uint_as_float(v[q]);
           __syncwarp();
-          const int lr0 = (warp & 3) * 32;
-          for (int i = 0; i < 32; ++i) {
-            bool li;
-            size_t bi;
-            const int ll = line_of(tile, lr0 + i, li, bi);
-            if (!li) continue;
-            const float val = tb[i * 33 + lane];
-            if (MODE == 0) {
-              static_cast<float*>(p.dst)[(size_t)ll * n + c0 + lane] = val;
-            } else {
-              double* dp = static_cast<double*>(p.dst) + bi + c0 + lane;
-              const double xv = (double)val * p.normfft;
-              *dp = ADD ? *dp + xv : xv;
+#pragma unroll 1
+          for (int i0 = 0; i0 < 32; i0 += 8) {
+            int b[8];
+            double old[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              b[u] = __shfl_sync(0xffffffffu, eb, i0 + u);
+              if (ADD) old[u] = b[u] >= 0 ? static_cast<double*>(p.dst)[b[u] + c0 + lane] : 0.;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+              if (b[u] < 0) continue;
+              const float val = tb[(i0 + u) * 33 + lane];
+              if (MODE == 0) {
+                static_cast<float*>(p.dst)[b[u] + c0 + lane] = val;
+              } else {
+                const double xv = (double)val * p.normfft;
+                static_cast<double*>(p.dst)[b[u] + c0 + lane] = ADD ? old[u] + xv : xv;
+              }
             }
           }
           __syncwarp();
         }
       }
-      (void)el;
     }
     tc_before();
     __syncthreads();
@@ -449,7 +504,7 @@ std::vector<uint16_t> xform_bmat(int kind, int dir, int n) {
 
 bool xform_gemm_length(int n) { return n == 64 || n == 128 || n == 256; }
 
-size_t xform_gemm_smem(int n) { return (size_t)GST * (2 * GM * GKC * 2 + 2 * (size_t)n * GKC * 2) + 8 * 8 + 16; }
+size_t xform_gemm_smem(int n) { return (size_t)GST * (2 * (GM / 8) * GSBO + 2 * (size_t)n * GKC * 2) + 8 * 8 + 16; }
 
 template <int MODE, bool ADD>
 static int set_attr_one(int n) {
