@@ -1720,11 +1720,11 @@ struct ZSolvePart {
     T* red = tile + (size_t)nz * NC;               // [2P][4][NC]: sub, diag, sup, rhs of the reduced rows
     T* xb = red + (size_t)8 * P * NC;              // [2P][NC]: x_s, x_e of every chunk
     const bool serial0 = zsing && __ldg(lam) == 0.;
-    if (bk.x == bk.nx - 1) {  // the extra block
+    if (bk.x == 0) {  // the extra block, first: its chain is the longest (as the last one: 94 -> 101 us at 256^3)
       if (serial0) zsolve_serial0<T>(ncol, nz, a, b, c, piv0, df0, work, zsing, tile);
       return;
     }
-    const int col0 = bk.x * NC, cols = EXACT ? NC : min(NC, ncol - col0);
+    const int col0 = (bk.x - 1) * NC, cols = EXACT ? NC : min(NC, ncol - col0);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int base = EXACT ? CH : nz / P, rem = EXACT ? 0 : nz % P;
     const int len = EXACT ? CH : base + (w < rem ? 1 : 0);
@@ -2172,7 +2172,7 @@ template <typename T, int CH, int P, bool EXACT>
 static void z_part_go(const Launch& Lc, const Geo& g, const PoissonPlan& pl, const DevScalars* sc) {
   const int ncol = g.nx * g.ny;
   constexpr int MINB = P == 8 ? (sizeof(T) == 4 ? 4 : 2) : 1;
-  // the tiles of columns, and the block of the singular column
+  // the block of the singular column, and the tiles of columns
   kgo<ZSolvePart<T, CH, P, EXACT>, 32 * P, MINB>(Lc, k_zsolve_part<T, CH, P, EXACT>, (ncol + ZP_NC - 1) / ZP_NC + 1,
                                                  32 * P, zpart_smem<T>(g.nz, P), ncol, g.nz, pl.lam, pl.a, pl.b, pl.c,
                                                  zpiv0<T>(pl), zdf0<T>(pl), sc, wbuf<T>(pl), pl.zsing);
