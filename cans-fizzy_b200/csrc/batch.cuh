@@ -35,6 +35,19 @@ struct Blk {
 __device__ __forceinline__ Blk blk_here() {
   return Blk{(int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, (int)gridDim.x, (int)gridDim.y, (int)gridDim.z};
 }
+// The same as the prologue of a kernel launched by kgo_chain.  A step is a chain
+// of kernels, many of them a few microseconds long; launched with programmatic
+// serialization, the next kernel's blocks come onto the device while this one
+// runs and wait here, for every earlier kernel's completion and memory, before
+// they read anything.  The trigger that lets this kernel's successor do the same
+// follows that wait, so at most one kernel waits behind another.  Both are
+// no-ops in a plain launch, but not free: kernels of a point per thread in
+// blocks of 128 keep blk_here (fillps at 256^3 took 137 instead of 93 us).
+__device__ __forceinline__ Blk blk_chain() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  return blk_here();
+}
 
 // a flat, trivially copyable argument list
 template <int I, class T>
@@ -138,6 +151,36 @@ inline void kgo(const Launch& L, K k, dim3 grid, dim3 block, size_t smem, V&&...
     return;
   }
   k<<<grid, block, smem, L.st>>>(std::forward<V>(v)...);
+}
+// kgo for a kernel that begins with blk_chain
+template <class F, int NT, int MINB, class K, class... V>
+inline void kgo_chain(const Launch& L, K k, dim3 grid, dim3 block, size_t smem, V&&... v) {
+  // Programmatic serialization where this kernel or the one before it has at
+  // most one block per SM.  Between two large kernels it costs more than the
+  // launch gap: the SMs that finish first take more than their share of the
+  // waiting blocks (every launch: a step at 160^3 +3%, 90x50x70 +4%; this rule:
+  // 64x2x128 -10%, 32^3 -8%, 64^3 -4%, 96^3 -1.6%, 160^3 and 90x50x70 -0.5 and
+  // -1.7%).  Not in an ensemble's graph, whose branches fill the device.
+  if (L.prev_blocks && !L.batched && !L.rec) {
+    const long long blocks = (long long)grid.x * grid.y * grid.z, few = L.nsm > 0 ? L.nsm : 148;
+    const bool early = blocks <= few || *L.prev_blocks <= few;
+    *L.prev_blocks = blocks;
+    if (early) {
+      cudaLaunchAttribute at{};
+      at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      at.val.programmaticStreamSerializationAllowed = 1;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = grid;
+      cfg.blockDim = block;
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = L.st;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      cudaLaunchKernelEx(&cfg, k, std::forward<V>(v)...);
+      return;
+    }
+  }
+  kgo<F, NT, MINB>(L, k, grid, block, smem, std::forward<V>(v)...);
 }
 
 }  // namespace cansfz

@@ -217,6 +217,9 @@ struct Launch {
   // 1 while an ensemble graph is captured: other cases fill the GPU, so
   // kernels favour fewer, larger blocks
   int batched;
+  // blocks of the context's previous launch (kgo: which launches may come onto
+  // the device early); null: none do
+  long long* prev_blocks = nullptr;
   // set: launches are recorded for a batched replay instead of issued
   Recorder* rec = nullptr;
   // tunable launch shapes (cansfz_plan): blocks per SM that the z split of

@@ -72,6 +72,7 @@ struct cansfz_ctx {
   cudaStream_t st = nullptr;
   bool own_stream = false;
   Launch L{};
+  long long prev_blocks = 0;  // Launch::prev_blocks
   Geo g{};
   Phys ph{};
   int n[3]{};
@@ -804,6 +805,7 @@ int cansfz_create(const cansfz_params* prm, void* stream, cansfz_ctx** out) {
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&c->L.nsm, cudaDevAttrMultiProcessorCount, dev);
   c->L.st = c->st;
+  c->L.prev_blocks = &c->prev_blocks;
   poisson_set_attributes();
   tiles_set_attributes();
   momentum_set_attributes();

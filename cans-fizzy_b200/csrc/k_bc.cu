@@ -99,7 +99,7 @@ struct BcStage {
 };
 template <int STAGE>
 __global__ void k_bc_stage(Geo g, BcGroup grp, const DevScalars* __restrict__ sc) {
-  BcStage<STAGE>::run(blk_here(), g, grp, sc);
+  BcStage<STAGE>::run(blk_chain(), g, grp, sc);
 }
 
 // ---------------------------------------------------------------------------
@@ -185,7 +185,7 @@ struct BcAll {
   }
 };
 __global__ void k_bc_all(Geo g, BcGroup grp, const DevScalars* __restrict__ sc, int px, int py, int pz) {
-  BcAll::run(blk_here(), g, grp, sc, px, py, pz);
+  BcAll::run(blk_chain(), g, grp, sc, px, py, pz);
 }
 
 void launch_bc_group(const Launch& L, const Geo& g, const BcGroup& grp, const DevScalars* sc) {
@@ -219,18 +219,18 @@ void launch_bc_group(const Launch& L, const Geo& g, const BcGroup& grp, const De
       }
     if (one) {
       const long long n = (long long)planes[2] * NX * NY + (long long)planes[1] * NX * NZ + (long long)planes[0] * NY * NZ;
-      kgo<BcAll, 256, 1>(L, k_bc_all, dim3((unsigned)((n + tb - 1) / tb), grp.nf), tb, 0, g, grp, sc, planes[0],
+      kgo_chain<BcAll, 256, 1>(L, k_bc_all, dim3((unsigned)((n + tb - 1) / tb), grp.nf), tb, 0, g, grp, sc, planes[0],
                          planes[1], planes[2]);
       return;
     }
   }
   if (any_per) {
     const int n = 2 * NX * NZ + 2 * NX * NY;
-    kgo<BcStage<ST_PER>, 256, 1>(L, k_bc_stage<ST_PER>, dim3((n + tb - 1) / tb, grp.nf), tb, 0, g, grp, sc);
+    kgo_chain<BcStage<ST_PER>, 256, 1>(L, k_bc_stage<ST_PER>, dim3((n + tb - 1) / tb, grp.nf), tb, 0, g, grp, sc);
   }
-  if (any_x) kgo<BcStage<ST_X>, 256, 1>(L, k_bc_stage<ST_X>, dim3((NY * NZ + tb - 1) / tb, grp.nf), tb, 0, g, grp, sc);
-  if (any_y) kgo<BcStage<ST_Y>, 256, 1>(L, k_bc_stage<ST_Y>, dim3((NX * NZ + tb - 1) / tb, grp.nf), tb, 0, g, grp, sc);
-  if (any_z) kgo<BcStage<ST_Z>, 256, 1>(L, k_bc_stage<ST_Z>, dim3((NX * NY + tb - 1) / tb, grp.nf), tb, 0, g, grp, sc);
+  if (any_x) kgo_chain<BcStage<ST_X>, 256, 1>(L, k_bc_stage<ST_X>, dim3((NY * NZ + tb - 1) / tb, grp.nf), tb, 0, g, grp, sc);
+  if (any_y) kgo_chain<BcStage<ST_Y>, 256, 1>(L, k_bc_stage<ST_Y>, dim3((NX * NZ + tb - 1) / tb, grp.nf), tb, 0, g, grp, sc);
+  if (any_z) kgo_chain<BcStage<ST_Z>, 256, 1>(L, k_bc_stage<ST_Z>, dim3((NX * NY + tb - 1) / tb, grp.nf), tb, 0, g, grp, sc);
 }
 
 // updt_rhs_b, src/bound.f90:341-396 (c_or_f = 'c', so q = 0): add the BC

@@ -501,7 +501,7 @@ __global__ void __launch_bounds__(tile::Shape<TYV>::NT, 512 / tile::Shape<TYV>::
     const double* __restrict__ po, const TI* __restrict__ kappa, const double* __restrict__ s, const SurfSplit sp,
     TI* __restrict__ duo, TI* __restrict__ dvo, TI* __restrict__ dwo, double* __restrict__ uo,
     double* __restrict__ vo, double* __restrict__ wo, const __grid_constant__ HaloMaps maps, int wrap) {
-  MomentumTile<TI, TYV, OPT, STG>::run(blk_here(), g, ph, sc, kz, u, v, w, psi, psio, fx, fy, fz, p, po, kappa, s, sp,
+  MomentumTile<TI, TYV, OPT, STG>::run(blk_chain(), g, ph, sc, kz, u, v, w, psi, psio, fx, fy, fz, p, po, kappa, s, sp,
       duo, dvo, dwo, uo, vo, wo, maps, wrap);
 }
 
@@ -567,11 +567,11 @@ static void momentum_go(const Launch& L, const Geo& g, const Phys& ph, const Dev
     }
   }
   if (use_tma)
-    kgo<MomentumTile<TI, TYV, OPT, 1>, S::NT, 512 / S::NT>(L, k_momentum_tile<TI, TYV, OPT, 1>,
+    kgo_chain<MomentumTile<TI, TYV, OPT, 1>, S::NT, 512 / S::NT>(L, k_momentum_tile<TI, TYV, OPT, 1>,
         tile::grid_of<TYV>(g, kz), dim3(S::TX, S::TY), mom_smem<TI, TYV, 1>(), g, ph, sc, kz, u, v, w, psi, psio, fx,
         fy, fz, p, po, kappa, s, sp, duo, dvo, dwo, uo, vo, wo, maps, L.wrap);
   else
-    kgo<MomentumTile<TI, TYV, OPT, 0>, S::NT, 512 / S::NT>(L, k_momentum_tile<TI, TYV, OPT, 0>,
+    kgo_chain<MomentumTile<TI, TYV, OPT, 0>, S::NT, 512 / S::NT>(L, k_momentum_tile<TI, TYV, OPT, 0>,
         tile::grid_of<TYV>(g, kz), dim3(S::TX, S::TY), mom_smem<TI, TYV, 0>(), g, ph, sc, kz, u, v, w, psi, psio, fx,
         fy, fz, p, po, kappa, s, sp, duo, dvo, dwo, uo, vo, wo, maps, L.wrap);
 }

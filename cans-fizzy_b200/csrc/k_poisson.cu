@@ -416,7 +416,7 @@ template <typename T, bool FUSED, int MC, int LC>
 __global__ void __launch_bounds__(256) k_fft_x_fwd(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
     const double* __restrict__ src, const double* __restrict__ u, const double* __restrict__ v,
     const double* __restrict__ w, Phys ph, T* __restrict__ work, int Lrt) {
-  FftXFwd<T, FUSED, MC, LC>::run(blk_here(), g, pl, sc, src, u, v, w, ph, work, Lrt);
+  FftXFwd<T, FUSED, MC, LC>::run(blk_chain(), g, pl, sc, src, u, v, w, ph, work, Lrt);
 }
 
 // ADD: dst += normfft * x (refinement correction) instead of dst = normfft * x
@@ -484,7 +484,7 @@ struct FftXBwd {
 template <typename T, bool ADD, int MC, int LC>
 __global__ void __launch_bounds__(256) k_fft_x_bwd(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
     const T* __restrict__ work, double normfft, double* __restrict__ dst, int Lrt, int wrap) {
-  FftXBwd<T, ADD, MC, LC>::run(blk_here(), g, pl, sc, work, normfft, dst, Lrt, wrap);
+  FftXBwd<T, ADD, MC, LC>::run(blk_chain(), g, pl, sc, work, normfft, dst, Lrt, wrap);
 }
 
 // ---------------------------------------------------------------------------
@@ -625,7 +625,7 @@ template <typename T, bool FUSED, int R>
 __global__ void __launch_bounds__(256) k_fft_x_fwd_w(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
     const double* __restrict__ src, const double* __restrict__ u, const double* __restrict__ v,
     const double* __restrict__ w, Phys ph, T* __restrict__ work) {
-  FftXFwdW<T, FUSED, R>::run(blk_here(), g, pl, sc, src, u, v, w, ph, work);
+  FftXFwdW<T, FUSED, R>::run(blk_chain(), g, pl, sc, src, u, v, w, ph, work);
 }
 
 template <typename T, bool ADD, int R>
@@ -695,7 +695,7 @@ struct FftXBwdW {
 template <typename T, bool ADD, int R>
 __global__ void __launch_bounds__(256) k_fft_x_bwd_w(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
     const T* __restrict__ work, double normfft, double* __restrict__ dst, int wrap) {
-  FftXBwdW<T, ADD, R>::run(blk_here(), g, pl, sc, work, normfft, dst, wrap);
+  FftXBwdW<T, ADD, R>::run(blk_chain(), g, pl, sc, work, normfft, dst, wrap);
 }
 
 // ---------------------------------------------------------------------------
@@ -757,7 +757,7 @@ struct FftY {
 template <typename T, int DIR, int MC, int LC>
 __global__ void __launch_bounds__(256) k_fft_y(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
                                                T* __restrict__ work, int Lrt) {
-  FftY<T, DIR, MC, LC>::run(blk_here(), g, pl, sc, work, Lrt);
+  FftY<T, DIR, MC, LC>::run(blk_chain(), g, pl, sc, work, Lrt);
 }
 
 // ---------------------------------------------------------------------------
@@ -1020,7 +1020,7 @@ template <typename T, bool FUSED, int MC>
 __global__ void __launch_bounds__(FftX2Fwd<T, FUSED, MC>::NT, 3) k_fft_x2_fwd(Geo g, LinePlan pl,
     const DevScalars* __restrict__ sc, const double* __restrict__ src, const double* __restrict__ u,
     const double* __restrict__ v, const double* __restrict__ w, Phys ph, T* __restrict__ work) {
-  FftX2Fwd<T, FUSED, MC>::run(blk_here(), g, pl, sc, src, u, v, w, ph, work);
+  FftX2Fwd<T, FUSED, MC>::run(blk_chain(), g, pl, sc, src, u, v, w, ph, work);
 }
 
 template <typename T, bool ADD, int MC>
@@ -1110,14 +1110,14 @@ template <typename T, bool ADD, int MC>
 __global__ void __launch_bounds__(FftX2Bwd<T, ADD, MC>::NT, 4) k_fft_x2_bwd(Geo g, LinePlan pl,
     const DevScalars* __restrict__ sc, const T* __restrict__ work, double normfft, double* __restrict__ dst,
     int wrap) {
-  FftX2Bwd<T, ADD, MC>::run(blk_here(), g, pl, sc, work, normfft, dst, wrap);
+  FftX2Bwd<T, ADD, MC>::run(blk_chain(), g, pl, sc, work, normfft, dst, wrap);
 }
 
 template <typename T, int DIR, int MC>
 __global__ void __launch_bounds__(FftY2<T, DIR, MC>::NT, 3) k_fft_y2(Geo g, LinePlan pl,
                                                                    const DevScalars* __restrict__ sc,
                                                                    T* __restrict__ work) {
-  FftY2<T, DIR, MC>::run(blk_here(), g, pl, sc, work);
+  FftY2<T, DIR, MC>::run(blk_chain(), g, pl, sc, work);
 }
 
 // ---------------------------------------------------------------------------
@@ -1231,7 +1231,7 @@ template <typename T, int DIR>
 __global__ void __launch_bounds__(FftYW<T, DIR>::NT, 2) k_fft_y512(Geo g, LinePlan pl,
                                                                   const DevScalars* __restrict__ sc,
                                                                   T* __restrict__ work) {
-  FftYW<T, DIR>::run(blk_here(), g, pl, sc, work);
+  FftYW<T, DIR>::run(blk_chain(), g, pl, sc, work);
 }
 
 // x lines of 512 points: the forward transform of a halo field's interior (or,
@@ -1292,7 +1292,7 @@ template <typename T, bool FUSED>
 __global__ void __launch_bounds__(256, 2) k_fft_x512_fwd(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
     const double* __restrict__ src, const double* __restrict__ u, const double* __restrict__ v,
     const double* __restrict__ w, Phys ph, T* __restrict__ work) {
-  FftXWFwd<T, FUSED>::run(blk_here(), g, pl, sc, src, u, v, w, ph, work);
+  FftXWFwd<T, FUSED>::run(blk_chain(), g, pl, sc, src, u, v, w, ph, work);
 }
 
 template <typename T, bool ADD>
@@ -1355,7 +1355,7 @@ struct FftXWBwd {
 template <typename T, bool ADD>
 __global__ void __launch_bounds__(256, 2) k_fft_x512_bwd(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
     const T* __restrict__ work, double normfft, double* __restrict__ dst, int wrap) {
-  FftXWBwd<T, ADD>::run(blk_here(), g, pl, sc, work, normfft, dst, wrap);
+  FftXWBwd<T, ADD>::run(blk_chain(), g, pl, sc, work, normfft, dst, wrap);
 }
 
 // ---------------------------------------------------------------------------
@@ -1578,7 +1578,7 @@ struct ZSolveF {
 template <typename T>
 __global__ void __launch_bounds__(128) k_zsolve_f(int ncol, int nz, const double* __restrict__ a,
     const T* __restrict__ piv, const T* __restrict__ df, const DevScalars* __restrict__ sc, T* __restrict__ work) {
-  ZSolveF<T>::run(blk_here(), ncol, nz, a, piv, df, sc, work);
+  ZSolveF<T>::run(blk_chain(), ncol, nz, a, piv, df, sc, work);
 }
 
 template <typename T>
@@ -1600,7 +1600,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) k_zsolve(int ncol, int nz, const double* __restrict__ lam,
     const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
     const DevScalars* __restrict__ sc, T* __restrict__ work, int zsing) {
-  ZSolve<T>::run(blk_here(), ncol, nz, lam, a, b, c, sc, work, zsing);
+  ZSolve<T>::run(blk_chain(), ncol, nz, lam, a, b, c, sc, work, zsing);
 }
 
 // ---------------------------------------------------------------------------
@@ -1838,7 +1838,7 @@ __global__ void __launch_bounds__(32 * P, P == 8 ? (sizeof(T) == 4 ? 4 : 2) : 1)
     const double* __restrict__ lam, const double* __restrict__ a, const double* __restrict__ b,
     const double* __restrict__ c, const T* __restrict__ piv0, const T* __restrict__ df0,
     const DevScalars* __restrict__ sc, T* __restrict__ work, int zsing) {
-  ZSolvePart<T, CH, P, EXACT>::run(blk_here(), ncol, nz, lam, a, b, c, piv0, df0, sc, work, zsing);
+  ZSolvePart<T, CH, P, EXACT>::run(blk_chain(), ncol, nz, lam, a, b, c, piv0, df0, sc, work, zsing);
 }
 
 // periodic z: gaussel_periodic (src/solver.f90:107-149)
@@ -1877,7 +1877,7 @@ template <typename T>
 __global__ void __launch_bounds__(128) k_zsolve_periodic(int ncol, int nz, const double* __restrict__ lam,
     const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
     const DevScalars* __restrict__ sc, T* __restrict__ work, T* __restrict__ work2) {
-  ZSolvePeriodic<T>::run(blk_here(), ncol, nz, lam, a, b, c, sc, work, work2);
+  ZSolvePeriodic<T>::run(blk_chain(), ncol, nz, lam, a, b, c, sc, work, work2);
 }
 
 // periodic z with the precomputed factors (those of the first n-1 levels)
@@ -1914,7 +1914,7 @@ __global__ void __launch_bounds__(128) k_zsolve_periodic_f(int ncol, int nz, con
     const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
     const T* __restrict__ piv, const T* __restrict__ df, const DevScalars* __restrict__ sc, T* __restrict__ work,
     T* __restrict__ work2) {
-  ZSolvePeriodicF<T>::run(blk_here(), ncol, nz, lam, a, b, c, piv, df, sc, work, work2);
+  ZSolvePeriodicF<T>::run(blk_chain(), ncol, nz, lam, a, b, c, piv, df, sc, work, work2);
 }
 
 // ---------------------------------------------------------------------------
@@ -2046,10 +2046,10 @@ static void x_forward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl,
       using X = FftX2Fwd<T, true, MC>;
       const dim3 g2((nlines + X::L - 1) / X::L);
       if (fused)
-        kgo<FftX2Fwd<T, true, MC>, X::NT, 3>(Lc, k_fft_x2_fwd<T, true, MC>, g2, X::NT, 0, g, pl.px, sc, nullptr, u, v,
+        kgo_chain<FftX2Fwd<T, true, MC>, X::NT, 3>(Lc, k_fft_x2_fwd<T, true, MC>, g2, X::NT, 0, g, pl.px, sc, nullptr, u, v,
                                             w, *ph, wbuf<T>(pl));
       else
-        kgo<FftX2Fwd<T, false, MC>, X::NT, 3>(Lc, k_fft_x2_fwd<T, false, MC>, g2, X::NT, 0, g, pl.px, sc, src,
+        kgo_chain<FftX2Fwd<T, false, MC>, X::NT, 3>(Lc, k_fft_x2_fwd<T, false, MC>, g2, X::NT, 0, g, pl.px, sc, src,
                                              nullptr, nullptr, nullptr, pz, wbuf<T>(pl));
       return;
     }
@@ -2058,10 +2058,10 @@ static void x_forward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl,
     if (pl.px.kind == 0 && pl.lmode == 0) {
       const dim3 g5((nlines + kW - 1) / kW);
       if (fused)
-        kgo<FftXWFwd<T, true>, 256, 2>(Lc, k_fft_x512_fwd<T, true>, g5, 256, w512_smem<T>(true), g, pl.px, sc, nullptr,
+        kgo_chain<FftXWFwd<T, true>, 256, 2>(Lc, k_fft_x512_fwd<T, true>, g5, 256, w512_smem<T>(true), g, pl.px, sc, nullptr,
                                        u, v, w, *ph, wbuf<T>(pl));
       else
-        kgo<FftXWFwd<T, false>, 256, 2>(Lc, k_fft_x512_fwd<T, false>, g5, 256, w512_smem<T>(true), g, pl.px, sc, src,
+        kgo_chain<FftXWFwd<T, false>, 256, 2>(Lc, k_fft_x512_fwd<T, false>, g5, 256, w512_smem<T>(true), g, pl.px, sc, src,
                                         nullptr, nullptr, nullptr, pz, wbuf<T>(pl));
       return;
     }
@@ -2071,19 +2071,19 @@ static void x_forward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl,
       constexpr int R = MC / 32;
       const dim3 gw((nlines + 8 * kWarpLines - 1) / (8 * kWarpLines));
       if (fused)
-        kgo<FftXFwdW<T, true, R>, 256, 1>(Lc, k_fft_x_fwd_w<T, true, R>, gw, 256, 0, g, pl.px, sc, nullptr, u, v, w,
+        kgo_chain<FftXFwdW<T, true, R>, 256, 1>(Lc, k_fft_x_fwd_w<T, true, R>, gw, 256, 0, g, pl.px, sc, nullptr, u, v, w,
                                           *ph, wbuf<T>(pl));
       else
-        kgo<FftXFwdW<T, false, R>, 256, 1>(Lc, k_fft_x_fwd_w<T, false, R>, gw, 256, 0, g, pl.px, sc, src, nullptr,
+        kgo_chain<FftXFwdW<T, false, R>, 256, 1>(Lc, k_fft_x_fwd_w<T, false, R>, gw, 256, 0, g, pl.px, sc, src, nullptr,
                                            nullptr, nullptr, pz, wbuf<T>(pl));
       return;
     }
   }
   if (fused)
-    kgo<FftXFwd<T, true, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_fwd<T, true, MC, xL<T, MC>()>, grid, 256, smem, g,
+    kgo_chain<FftXFwd<T, true, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_fwd<T, true, MC, xL<T, MC>()>, grid, 256, smem, g,
                                                    pl.px, sc, nullptr, u, v, w, *ph, wbuf<T>(pl), L);
   else
-    kgo<FftXFwd<T, false, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_fwd<T, false, MC, xL<T, MC>()>, grid, 256, smem, g,
+    kgo_chain<FftXFwd<T, false, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_fwd<T, false, MC, xL<T, MC>()>, grid, 256, smem, g,
                                                     pl.px, sc, src, nullptr, nullptr, nullptr, pz, wbuf<T>(pl), L);
 }
 
@@ -2107,9 +2107,9 @@ static void y_pass_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl, co
       using Y = FftY2<T, 1, MC>;
       const dim3 g2((g.nx + Y::L - 1) / Y::L, g.nz);
       if (dir > 0)
-        kgo<FftY2<T, 1, MC>, Y::NT, 3>(Lc, k_fft_y2<T, 1, MC>, g2, Y::NT, 0, g, pl.py, sc, wbuf<T>(pl));
+        kgo_chain<FftY2<T, 1, MC>, Y::NT, 3>(Lc, k_fft_y2<T, 1, MC>, g2, Y::NT, 0, g, pl.py, sc, wbuf<T>(pl));
       else
-        kgo<FftY2<T, -1, MC>, Y::NT, 3>(Lc, k_fft_y2<T, -1, MC>, g2, Y::NT, 0, g, pl.py, sc, wbuf<T>(pl));
+        kgo_chain<FftY2<T, -1, MC>, Y::NT, 3>(Lc, k_fft_y2<T, -1, MC>, g2, Y::NT, 0, g, pl.py, sc, wbuf<T>(pl));
       return;
     }
   }
@@ -2117,9 +2117,9 @@ static void y_pass_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl, co
     if (pl.py.kind == 0 && pl.lmode == 0) {
       const dim3 g5((g.nx + kW - 1) / kW, g.nz);
       if (dir > 0)
-        kgo<FftYW<T, 1>, 256, 2>(Lc, k_fft_y512<T, 1>, g5, 256, w512_smem<T>(false), g, pl.py, sc, wbuf<T>(pl));
+        kgo_chain<FftYW<T, 1>, 256, 2>(Lc, k_fft_y512<T, 1>, g5, 256, w512_smem<T>(false), g, pl.py, sc, wbuf<T>(pl));
       else
-        kgo<FftYW<T, -1>, 256, 2>(Lc, k_fft_y512<T, -1>, g5, 256, w512_smem<T>(false), g, pl.py, sc, wbuf<T>(pl));
+        kgo_chain<FftYW<T, -1>, 256, 2>(Lc, k_fft_y512<T, -1>, g5, 256, w512_smem<T>(false), g, pl.py, sc, wbuf<T>(pl));
       return;
     }
   }
@@ -2127,10 +2127,10 @@ static void y_pass_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl, co
   const size_t smem = 4 * (size_t)m * (L | 1) * sizeof(T);
   const dim3 grid((g.nx + L - 1) / L, g.nz);
   if (dir > 0)
-    kgo<FftY<T, 1, MC, yL<T, MC>()>, 256, 1>(Lc, k_fft_y<T, 1, MC, yL<T, MC>()>, grid, 256, smem, g, pl.py, sc,
+    kgo_chain<FftY<T, 1, MC, yL<T, MC>()>, 256, 1>(Lc, k_fft_y<T, 1, MC, yL<T, MC>()>, grid, 256, smem, g, pl.py, sc,
                                              wbuf<T>(pl), L);
   else
-    kgo<FftY<T, -1, MC, yL<T, MC>()>, 256, 1>(Lc, k_fft_y<T, -1, MC, yL<T, MC>()>, grid, 256, smem, g, pl.py, sc,
+    kgo_chain<FftY<T, -1, MC, yL<T, MC>()>, 256, 1>(Lc, k_fft_y<T, -1, MC, yL<T, MC>()>, grid, 256, smem, g, pl.py, sc,
                                               wbuf<T>(pl), L);
 }
 
@@ -2173,7 +2173,7 @@ static void z_part_go(const Launch& Lc, const Geo& g, const PoissonPlan& pl, con
   const int ncol = g.nx * g.ny;
   constexpr int MINB = P == 8 ? (sizeof(T) == 4 ? 4 : 2) : 1;
   // the block of the singular column, and the tiles of columns
-  kgo<ZSolvePart<T, CH, P, EXACT>, 32 * P, MINB>(Lc, k_zsolve_part<T, CH, P, EXACT>, (ncol + ZP_NC - 1) / ZP_NC + 1,
+  kgo_chain<ZSolvePart<T, CH, P, EXACT>, 32 * P, MINB>(Lc, k_zsolve_part<T, CH, P, EXACT>, (ncol + ZP_NC - 1) / ZP_NC + 1,
                                                  32 * P, zpart_smem<T>(g.nz, P), ncol, g.nz, pl.lam, pl.a, pl.b, pl.c,
                                                  zpiv0<T>(pl), zdf0<T>(pl), sc, wbuf<T>(pl), pl.zsing);
 }
@@ -2214,20 +2214,20 @@ static void z_pass(const Launch& Lc, const Geo& g, const PoissonPlan& pl, const 
   }
   if (zpiv<T>(pl) && zdf<T>(pl)) {
     if (pl.zper)
-      kgo<ZSolvePeriodicF<T>, 128, 1>(Lc, k_zsolve_periodic_f<T>, (ncol + tb - 1) / tb, tb, 0, ncol, g.nz, pl.lam,
+      kgo_chain<ZSolvePeriodicF<T>, 128, 1>(Lc, k_zsolve_periodic_f<T>, (ncol + tb - 1) / tb, tb, 0, ncol, g.nz, pl.lam,
                                       pl.a, pl.b, pl.c, zpiv<T>(pl), zdf<T>(pl), sc, wbuf<T>(pl), wbuf2<T>(pl));
     else
-      kgo<ZSolveF<T>, 128, 1>(Lc, k_zsolve_f<T>, (ncol + tb - 1) / tb, tb, 0, ncol, g.nz, pl.a, zpiv<T>(pl),
+      kgo_chain<ZSolveF<T>, 128, 1>(Lc, k_zsolve_f<T>, (ncol + tb - 1) / tb, tb, 0, ncol, g.nz, pl.a, zpiv<T>(pl),
                               zdf<T>(pl), sc, wbuf<T>(pl));
     return;
   }
   const int nch = (g.nz + ZCH - 1) / ZCH;
   const size_t smem = (size_t)nch * tb * sizeof(T);
   if (pl.zper)
-    kgo<ZSolvePeriodic<T>, 128, 1>(Lc, k_zsolve_periodic<T>, (ncol + tb - 1) / tb, tb, smem, ncol, g.nz, pl.lam,
+    kgo_chain<ZSolvePeriodic<T>, 128, 1>(Lc, k_zsolve_periodic<T>, (ncol + tb - 1) / tb, tb, smem, ncol, g.nz, pl.lam,
                                    pl.a, pl.b, pl.c, sc, wbuf<T>(pl), wbuf2<T>(pl));
   else
-    kgo<ZSolve<T>, 128, 1>(Lc, k_zsolve<T>, (ncol + tb - 1) / tb, tb, smem, ncol, g.nz, pl.lam, pl.a, pl.b, pl.c,
+    kgo_chain<ZSolve<T>, 128, 1>(Lc, k_zsolve<T>, (ncol + tb - 1) / tb, tb, smem, ncol, g.nz, pl.lam, pl.a, pl.b, pl.c,
                            sc, wbuf<T>(pl), pl.zsing);
 }
 
@@ -2241,14 +2241,14 @@ static void x_backward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl
   if constexpr (y2_length(MC)) {
     if (pl.px.kind == 0 && pl.lmode == 0) {
       using X = FftX2Bwd<T, ADD, MC>;
-      kgo<FftX2Bwd<T, ADD, MC>, X::NT, 4>(Lc, k_fft_x2_bwd<T, ADD, MC>, (nlines + X::L - 1) / X::L, X::NT, 0, g,
+      kgo_chain<FftX2Bwd<T, ADD, MC>, X::NT, 4>(Lc, k_fft_x2_bwd<T, ADD, MC>, (nlines + X::L - 1) / X::L, X::NT, 0, g,
                                          pl.px, sc, wbuf<T>(pl), pl.normfft, dst, ADD ? 0 : Lc.wrap);
       return;
     }
   }
   if constexpr (MC == 256) {
     if (pl.px.kind == 0 && pl.lmode == 0) {
-      kgo<FftXWBwd<T, ADD>, 256, 2>(Lc, k_fft_x512_bwd<T, ADD>, (nlines + kW - 1) / kW, 256, w512_smem<T>(true), g,
+      kgo_chain<FftXWBwd<T, ADD>, 256, 2>(Lc, k_fft_x512_bwd<T, ADD>, (nlines + kW - 1) / kW, 256, w512_smem<T>(true), g,
                                     pl.px, sc, wbuf<T>(pl), pl.normfft, dst, ADD ? 0 : Lc.wrap);
       return;
     }
@@ -2256,12 +2256,12 @@ static void x_backward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl
   if constexpr (MC == 64 || MC == 128) {
     if (pl.px.kind == 0) {
       constexpr int R = MC / 32;
-      kgo<FftXBwdW<T, ADD, R>, 256, 1>(Lc, k_fft_x_bwd_w<T, ADD, R>, (nlines + 8 * kWarpLines - 1) / (8 * kWarpLines),
+      kgo_chain<FftXBwdW<T, ADD, R>, 256, 1>(Lc, k_fft_x_bwd_w<T, ADD, R>, (nlines + 8 * kWarpLines - 1) / (8 * kWarpLines),
                                        256, 0, g, pl.px, sc, wbuf<T>(pl), pl.normfft, dst, ADD ? 0 : Lc.wrap);
       return;
     }
   }
-  kgo<FftXBwd<T, ADD, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_bwd<T, ADD, MC, xL<T, MC>()>, (nlines + L - 1) / L, 256,
+  kgo_chain<FftXBwd<T, ADD, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_bwd<T, ADD, MC, xL<T, MC>()>, (nlines + L - 1) / L, 256,
                                                 smem, g, pl.px, sc, wbuf<T>(pl), pl.normfft, dst, L,
                                                 ADD ? 0 : Lc.wrap);
 }

@@ -205,15 +205,15 @@ struct CmptPhi {
 template <bool ACDI, typename TO>
 __global__ void k_cmpt_phi(int n, const DevScalars* __restrict__ sc, const double* __restrict__ psi,
                            TO* __restrict__ phi) {
-  CmptPhi<ACDI, TO>::run(blk_here(), n, sc, psi, phi);
+  CmptPhi<ACDI, TO>::run(blk_chain(), n, sc, psi, phi);
 }
 
 void launch_cmpt_phi(const Launch& L, const Geo& g, const DevScalars* sc, bool acdi, const double* psi,
                      double* phi) {
   const int n = g.hsize();
   const int nb = (n + 256 * kPhiPer - 1) / (256 * kPhiPer);
-  if (acdi) kgo<CmptPhi<true, double>, 256, 1>(L, k_cmpt_phi<true, double>, nb, 256, 0, n, sc, psi, phi);
-  else kgo<CmptPhi<false, double>, 256, 1>(L, k_cmpt_phi<false, double>, nb, 256, 0, n, sc, psi, phi);
+  if (acdi) kgo_chain<CmptPhi<true, double>, 256, 1>(L, k_cmpt_phi<true, double>, nb, 256, 0, n, sc, psi, phi);
+  else kgo_chain<CmptPhi<false, double>, 256, 1>(L, k_cmpt_phi<false, double>, nb, 256, 0, n, sc, psi, phi);
 }
 // the mixed form: phi evaluated in FP64 and stored in FP32
 // (narrow_only: Youngs without SDF normals works on psi itself, stored in FP32)
@@ -234,10 +234,10 @@ void launch_cmpt_phi_f32(const Launch& L, const Geo& g, const DevScalars* sc, bo
   const int n = g.hsize();
   if (narrow_only) kgo<Narrow, 256, 1>(L, k_narrow, (n + 255) / 256, 256, 0, n, sc, psi, phi);
   else if (acdi)
-    kgo<CmptPhi<true, float>, 256, 1>(L, k_cmpt_phi<true, float>, (n + 256 * kPhiPer - 1) / (256 * kPhiPer), 256, 0,
+    kgo_chain<CmptPhi<true, float>, 256, 1>(L, k_cmpt_phi<true, float>, (n + 256 * kPhiPer - 1) / (256 * kPhiPer), 256, 0,
                                       n, sc, psi, phi);
   else
-    kgo<CmptPhi<false, float>, 256, 1>(L, k_cmpt_phi<false, float>, (n + 256 * kPhiPer - 1) / (256 * kPhiPer), 256,
+    kgo_chain<CmptPhi<false, float>, 256, 1>(L, k_cmpt_phi<false, float>, (n + 256 * kPhiPer - 1) / (256 * kPhiPer), 256,
                                        0, n, sc, psi, phi);
 }
 
@@ -851,12 +851,12 @@ __global__ void __launch_bounds__(256) k_correc_updatep(Geo g, Phys ph, const De
                                                         double* __restrict__ v, double* __restrict__ w,
                                                         const double* __restrict__ pp, double* __restrict__ pout,
                                                         int wrap) {
-  CorrecUpdatep::run(blk_here(), g, ph, sc, p, u, v, w, pp, pout, wrap);
+  CorrecUpdatep::run(blk_chain(), g, ph, sc, p, u, v, w, pp, pout, wrap);
 }
 void launch_correc_updatep(const Launch& L, const Geo& g, const Phys& ph, const DevScalars* sc, const double* p,
                            double* u, double* v, double* w, const double* pp, double* pout) {
   const dim3 b(32, 8), gr((g.nx + 2 + 31) / 32, (g.ny + 2 + 7) / 8, (g.nz + 2 + kCorrecLevels - 1) / kCorrecLevels);
-  kgo<CorrecUpdatep, 256, 1>(L, k_correc_updatep, gr, b, 0, g, ph, sc, p, u, v, w, pp, pout, L.wrap);
+  kgo_chain<CorrecUpdatep, 256, 1>(L, k_correc_updatep, gr, b, 0, g, ph, sc, p, u, v, w, pp, pout, L.wrap);
 }
 
 // updatep, src/updatep.f90:13-24
@@ -1249,7 +1249,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_step_reduce(Geo g, DevScalar
                                                                 const double* __restrict__ u,
                                                                 const double* __restrict__ v,
                                                                 const double* __restrict__ w) {
-  StepReduce::run(blk_here(), g, sc, acdi, part, u, v, w);
+  StepReduce::run(blk_chain(), g, sc, acdi, part, u, v, w);
 }
 struct StepReduceFinal {
   static __device__ __forceinline__ void run(const Blk& bk, const Phys& ph, DevScalars* __restrict__ sc, int nb,
@@ -1273,7 +1273,7 @@ struct StepReduceFinal {
   }
 };
 __global__ void k_step_reduce_final(Phys ph, DevScalars* __restrict__ sc, int nb, const double* __restrict__ part) {
-  StepReduceFinal::run(blk_here(), ph, sc, nb, part);
+  StepReduceFinal::run(blk_chain(), ph, sc, nb, part);
 }
 void launch_step_reductions(const Launch& L, const Geo& g, const Phys& ph, DevScalars* sc, double* partial,
                             const double* u, const double* v, const double* w) {
@@ -1283,8 +1283,8 @@ void launch_step_reductions(const Launch& L, const Geo& g, const Phys& ph, DevSc
   // 0.096 ms at 256^3)
   int nb = (L.nsm > 0 ? L.nsm : 148) * 4;
   if (nb > nrows) nb = nrows;
-  kgo<StepReduce, 256, 1>(L, k_step_reduce, nb, kReduceThreads, 0, g, sc, ph.acdi, partial, u, v, w);
-  kgo<StepReduceFinal, 1024, 1>(L, k_step_reduce_final, 1, 1024, 0, ph, sc, nb, partial);
+  kgo_chain<StepReduce, 256, 1>(L, k_step_reduce, nb, kReduceThreads, 0, g, sc, ph.acdi, partial, u, v, w);
+  kgo_chain<StepReduceFinal, 1024, 1>(L, k_step_reduce_final, 1, 1024, 0, ph, sc, nb, partial);
 }
 
 // bulk_mean_12_stag, src/utils.f90:68-136
@@ -1376,10 +1376,10 @@ struct StepBegin {
   }
 };
 __global__ void k_step_begin(DevScalars* sc, int icheck) {
-  StepBegin::run(blk_here(), sc, icheck);
+  StepBegin::run(blk_chain(), sc, icheck);
 }
 void launch_step_begin(const Launch& L, DevScalars* sc, int icheck) {
-  kgo<StepBegin, 1, 1>(L, k_step_begin, 1, 1, 0, sc, icheck);
+  kgo_chain<StepBegin, 1, 1>(L, k_step_begin, 1, 1, 0, sc, icheck);
 }
 struct StepEnd {
   static __device__ __forceinline__ void run(const Blk& bk, DevScalars* sc) {
@@ -1391,11 +1391,11 @@ struct StepEnd {
   }
 };
 __global__ void k_step_end(DevScalars* sc) {
-  StepEnd::run(blk_here(), sc);
+  StepEnd::run(blk_chain(), sc);
 }
 void launch_step_end(const Launch& L, const Phys& ph, DevScalars* sc) {
   (void)ph;
-  kgo<StepEnd, 1, 1>(L, k_step_end, 1, 1, 0, sc);
+  kgo_chain<StepEnd, 1, 1>(L, k_step_end, 1, 1, 0, sc);
 }
 
 }  // namespace cansfz

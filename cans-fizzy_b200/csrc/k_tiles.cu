@@ -197,7 +197,7 @@ __global__ void __launch_bounds__(tile::Shape<TYV>::NT + tile::Shape<TYV>::TX, 4
                                                           const TI* __restrict__ phi, TI* __restrict__ normx,
                                                           TI* __restrict__ normy, TI* __restrict__ normz,
                                                           TI* __restrict__ kappa, int wrap) {
-  YoungsTile<TI, TYV>::run(blk_here(), g, sc, kz, phi, normx, normy, normz, kappa, wrap);
+  YoungsTile<TI, TYV>::run(blk_chain(), g, sc, kz, phi, normx, normy, normz, kappa, wrap);
 }
 
 // ---------------------------------------------------------------------------
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(tile::Shape<TYV>::TX * (tile::Shape<TYV>::TY +
     const TI* __restrict__ nx_, const TI* __restrict__ ny_, const TI* __restrict__ nz_,
     const TI* __restrict__ phi, const double* __restrict__ psi, TI* __restrict__ dpsidt,
     TI* __restrict__ fx, TI* __restrict__ fy, TI* __restrict__ fz, double* __restrict__ psi_out, int wrap) {
-  AcdiTile<TI, SDF, UPD, TYV>::run(blk_here(), g, sc, kz, u, v, w, nx_, ny_, nz_, phi, psi, dpsidt, fx, fy, fz,
+  AcdiTile<TI, SDF, UPD, TYV>::run(blk_chain(), g, sc, kz, u, v, w, nx_, ny_, nz_, phi, psi, dpsidt, fx, fy, fz,
       psi_out, wrap);
 }
 
@@ -420,7 +420,7 @@ static void youngs_go(const Launch& L, const Geo& g, const DevScalars* sc, const
                       TI* kappa) {
   using S = tile::Shape<TYV>;
   const int kz = tile::kz_of<TYV>(g, L.batched, L.nsm, L.phase_slots > 0 ? L.phase_slots : 24, TYV == 8 ? 4 : 8);
-  kgo<YoungsTile<TI, TYV>, S::NT + S::TX, 4>(L, k_youngs_tile<TI, TYV>, tile::grid_of<TYV>(g, kz),
+  kgo_chain<YoungsTile<TI, TYV>, S::NT + S::TX, 4>(L, k_youngs_tile<TI, TYV>, tile::grid_of<TYV>(g, kz),
                                               dim3(S::TX, S::TY + 1), 0, g, sc, kz, phi, nx, ny, nz, kappa, L.wrap);
 }
 
@@ -437,7 +437,7 @@ static void acdi_go(const Launch& L, const Geo& g, const DevScalars* sc, const d
                     double* psi_out, TI* hist, TI* fx, TI* fy, TI* fz) {
   using S = tile::Shape<TYV>;
   const int kz = tile::kz_of<TYV>(g, L.batched, L.nsm, L.phase_slots > 0 ? L.phase_slots : 24, TYV == 8 ? 3 : 6);
-  kgo<AcdiTile<TI, SDF, UPD, TYV>, S::TX * (S::TY + 1), 3>(L, k_acdi_tile<TI, SDF, UPD, TYV>,
+  kgo_chain<AcdiTile<TI, SDF, UPD, TYV>, S::TX * (S::TY + 1), 3>(L, k_acdi_tile<TI, SDF, UPD, TYV>,
                                              tile::grid_of<TYV>(g, kz),
                                              dim3(S::TX, S::TY + 1), acdi_smem<TI, SDF, TYV>(), g, sc, kz, u, v, w, nx,
                                              ny, nz, phi, psi, hist, fx, fy, fz, psi_out, L.wrap);
