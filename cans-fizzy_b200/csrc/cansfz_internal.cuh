@@ -214,8 +214,8 @@ struct Recorder;  // batch.cuh
 struct Launch {
   cudaStream_t st;
   int nsm;
-  // 1 while an ensemble graph is captured: other cases fill the GPU, so
-  // kernels favour fewer, larger blocks
+  // not 0 while an ensemble's step is captured or recorded: the z levels per
+  // block of the tile kernels, which there do not split z to fill the GPU
   int batched;
   // blocks of the context's previous launch (kgo: which launches may come onto
   // the device early); null: none do

@@ -732,12 +732,12 @@ void enqueue_step(cansfz_ctx* c, const StageMark* mk = nullptr) {
 // One step of case c recorded instead of issued.  Launches that do not go
 // through the recorder are caught by a throwaway stream capture: the record
 // is complete (the step can be replayed batched) when that capture is empty.
-int record_step(cansfz_ctx* c, Recorder* rec, bool* complete) {
+int record_step(cansfz_ctx* c, Recorder* rec, bool* complete, int levels) {
   *complete = false;
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
   c->L.rec = rec;
-  c->L.batched = 1;
+  c->L.batched = levels;
   enqueue_step(c);
   c->L.rec = nullptr;
   c->L.batched = 0;
@@ -748,6 +748,18 @@ int record_step(cansfz_ctx* c, Recorder* rec, bool* complete) {
   CK(e);
   *complete = nodes == 0 && !rec->e.empty();
   return CANSFZ_OK;
+}
+
+// Levels per block of the tile kernels in an ensemble's step.  32 levels spend
+// 6% on the planes a block loads beyond its own (8 levels: 25%), which is what
+// counts when the cases fill the GPU; with less work their latency does, one
+// level after the other.  Per pass of 8 steps with 32 -> 8 levels: 12 2-D and 12
+// 3-D cases (11.5 million cells) 20.9 -> 21.1 ms, 12 2-D ones (1.1 million) 6.1 ->
+// 5.6 ms, 4 and 4 (4 million) 5.3 -> 4.6 ms.
+int ensemble_levels(const std::vector<cansfz_ctx*>& cases) {
+  double cells = 0.;
+  for (const cansfz_ctx* c : cases) cells += (double)c->g.tsize();
+  return cells < 8e6 ? 8 : 32;
 }
 
 bool same_record(const Recorder& a, const Recorder& b) {
@@ -1170,6 +1182,7 @@ int cansfz_ensemble_step(cansfz_ensemble* e, int nsteps, int* status_out) {
       // record every case's step; cases whose records agree launch for
       // launch (same kernels, grids and shared memory: same sizes and
       // options) form a group that is replayed as batched launches
+      const int levels = ensemble_levels(e->cases);
       std::vector<Recorder> rec(n);
       std::vector<std::vector<int>> groups;
       // branches in order of decreasing size, so that the longest steps
@@ -1182,7 +1195,7 @@ int cansfz_ensemble_step(cansfz_ensemble* e, int nsteps, int* status_out) {
       for (int q : order) {
         bool complete = false;
         if (e->batch > 1) {
-          if (int rc = record_step(e->cases[q], &rec[q], &complete)) return rc;
+          if (int rc = record_step(e->cases[q], &rec[q], &complete, levels)) return rc;
         }
         bool placed = false;
         for (auto& gr : groups)
@@ -1251,7 +1264,7 @@ int cansfz_ensemble_step(cansfz_ensemble* e, int nsteps, int* status_out) {
         cudaStream_t bs = c0->st;
         CK(cudaStreamWaitEvent(bs, e->fork, 0));
         if (gr.size() == 1) {
-          c0->L.batched = 1;
+          c0->L.batched = levels;
           enqueue_step(c0);
           c0->L.batched = 0;
         } else {

@@ -63,9 +63,8 @@ inline int rows_of(const Geo& g) { return g.ny <= 2 ? 2 : 8; }
 template <int TYV>
 inline int kz_of(const Geo& g, int batched, int nsm, int slots, int res) {
   using S = Shape<TYV>;
-  // in an ensemble the other cases keep the GPU busy: 32 levels per block
-  // spend 6% on the two extra planes each block loads (25% at 8 levels)
-  if (batched) return g.nz < 32 ? g.nz : 32;
+  // in an ensemble the other cases keep the GPU busy
+  if (batched) return g.nz < batched ? g.nz : batched;
   // several waves of resident blocks on each of the device's SMs (148 on a
   // B200), so the last partial wave costs little; at least 8 levels per
   // block (each block loads two planes and evaluates one face/vertex plane
