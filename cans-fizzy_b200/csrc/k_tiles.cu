@@ -94,14 +94,11 @@ struct YoungsTile {
 
     // cell plane kk (kb-1 <= kk <= ke+1) into its ring slot; an empty group
     // past the top keeps the wait counts uniform
+    const PlaneCopy<PX, PXY, NTT> cells(g, i0, j0, tid);
     auto issue = [&](int kk) {
       if (kk <= ke + 1) {
         T* dst = pl[kk % NCP];
-        for (int q = tid; q < PXY; q += NTT) {
-          int h;
-          const bool ok = plane_cell<PX>(g, i0, j0, kk, q, &h);
-          cp_async(dst + q, phi + (ok ? h : 0), ok);
-        }
+        cells.each(kk * g.sxy, [&](int q, int h, bool ok) { cp_async(dst + q, phi + h, ok); });
       }
       cp_commit();
     };
@@ -268,7 +265,6 @@ struct AcdiTile {
     const int tx = threadIdx.x, ty = threadIdx.y, tid = tx + TX * ty;
     const int i0 = bk.x * TX + 1, j0 = bk.y * TY + 1;
     const int kb = bk.z * kz + 1, ke = min(kb + kz - 1, g.nz);
-    const int sx = g.sx;
     AcdiCoef<T> cf;
     cf.gam = (T)sc->gam;
     const T seps = (T)sc->seps;
@@ -278,18 +274,19 @@ struct AcdiTile {
     const T dxi = (T)g.dxi, dyi = (T)g.dyi;
     const bool first2 = sc->first_rk2fl;
 
-    auto issue = [&](int kk) {
-      const int s = kk % NSLOT;
-      for (int q = tid; q < PXY; q += NTA) {
-        int h;
-        const bool ok = plane_cell<PX>(g, i0, j0, kk, q, &h);
-        const int hh = ok ? h : 0;
-        cp_async(s_psi + s * PXY + q, psi + hh, ok);
-        cp_async(s_n + (s * 3 + 0) * PXY + q, nx_ + hh, ok);
-        cp_async(s_n + (s * 3 + 1) * PXY + q, ny_ + hh, ok);
-        cp_async(s_n + (s * 3 + 2) * PXY + q, nz_ + hh, ok);
-        if (SDF) cp_async(s_phi + s * PXY + q, phi + hh, ok);
-      }
+    const PlaneCopy<PX, PXY, NTA> cells(g, i0, j0, tid);
+    // plane kk into ring slot s
+    auto issue = [&](int kk, int s) {
+      double* dp = s_psi + s * PXY;
+      T* dn = s_n + s * 3 * PXY;
+      T* df = s_phi + s * PXY;
+      cells.each(kk * g.sxy, [&](int q, int hh, bool ok) {
+        cp_async(dp + q, psi + hh, ok);
+        cp_async(dn + q, nx_ + hh, ok);
+        cp_async(dn + PXY + q, ny_ + hh, ok);
+        cp_async(dn + 2 * PXY + q, nz_ + hh, ok);
+        if (SDF) cp_async(df + q, phi + hh, ok);
+      });
       cp_commit();
     };
     // face between plane elements qa (slot sa) and qb (slot sb)
@@ -305,14 +302,16 @@ struct AcdiTile {
     const bool act = ty < TY && i <= g.nx && j <= g.ny;
     const int qc = (tx + 1) + PX * (ty + 1);  // the thread's own cell in a plane
 
-    issue(kb - 1);
-    issue(kb);
-    issue(kb + 1);
+    const int wox = wrap_ox(g, wrap, i), woy = wrap_oy(g, wrap, j);  // the column's x and y images
+    int s0 = 1, s1 = 2, s2 = 0;  // ring slots of planes k, k+1 and k+2
+    issue(kb - 1, 0);
+    issue(kb, 1);
+    issue(kb + 1, 2);
     cp_wait<1>();
     __syncthreads();
     T up_zm = T(0), rg_zm = T(0);
     if (act)
-      face(2, (T)g.dzci[kb - 1], (kb - 1) % NSLOT, qc, kb % NSLOT, qc, (T)__ldg(w + g.h(i, j, kb - 1)), &up_zm,
+      face(2, (T)g.dzci[kb - 1], s2, qc, s0, qc, (T)__ldg(w + g.h(i, j, kb - 1)), &up_zm,
            &rg_zm);
     __syncthreads();  // plane kb-1's slot is refilled next
 
@@ -322,11 +321,10 @@ struct AcdiTile {
       vx_n = (T)__ldg(u + c); vy_n = (T)__ldg(v + c); vz_n = (T)__ldg(w + c);
     }
     for (int k = kb; k <= ke; ++k) {
-      if (k + 2 <= ke + 1) issue(k + 2);
+      if (k + 2 <= ke + 1) issue(k + 2, s2);
       else cp_commit();
       cp_wait<1>();
       __syncthreads();  // plane k+1 is in; every thread is done with level k-1
-      const int s0 = k % NSLOT, s1 = (k + 1) % NSLOT;
       T up_zp = T(0), rg_zp = T(0);
       T dO_pre = T(0);
       if (act) {
@@ -389,7 +387,7 @@ struct AcdiTile {
         fx[c] = ex;
         fy[c] = ey;
         fz[c] = ez;
-        store_wraps(g, wrap, i, j, k, [&](int h) {
+        store_images(c, wox, woy, wrap_oz(g, wrap, k), [&](int h) {
           if (UPD) psi_out[h] = pn;
           fx[h] = ex;
           fy[h] = ey;
@@ -398,12 +396,18 @@ struct AcdiTile {
       }
       up_zm = up_zp;
       rg_zm = rg_zp;
+      const int sk = s0;
+      s0 = s1;
+      s1 = s2;
+      s2 = sk;
     }
-    (void)sx;
   }
 };
+// blocks per SM: three in FP64, four in FP32 (56 registers, as many as it needs)
+template <typename TI>
+constexpr int acdi_blocks() { return sizeof(TI) == 8 ? 3 : 4; }
 template <typename TI, bool SDF, bool UPD, int TYV>
-__global__ void __launch_bounds__(tile::Shape<TYV>::TX * (tile::Shape<TYV>::TY + 1), 3) k_acdi_tile(Geo g, const DevScalars* __restrict__ sc, int kz,
+__global__ void __launch_bounds__(tile::Shape<TYV>::TX * (tile::Shape<TYV>::TY + 1), acdi_blocks<TI>()) k_acdi_tile(Geo g, const DevScalars* __restrict__ sc, int kz,
     const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ w,
     const TI* __restrict__ nx_, const TI* __restrict__ ny_, const TI* __restrict__ nz_,
     const TI* __restrict__ phi, const double* __restrict__ psi, TI* __restrict__ dpsidt,
@@ -437,7 +441,7 @@ static void acdi_go(const Launch& L, const Geo& g, const DevScalars* sc, const d
                     double* psi_out, TI* hist, TI* fx, TI* fy, TI* fz) {
   using S = tile::Shape<TYV>;
   const int kz = tile::kz_of<TYV>(g, L.batched, L.nsm, L.phase_slots > 0 ? L.phase_slots : 24, TYV == 8 ? 3 : 6);
-  kgo_chain<AcdiTile<TI, SDF, UPD, TYV>, S::TX * (S::TY + 1), 3>(L, k_acdi_tile<TI, SDF, UPD, TYV>,
+  kgo_chain<AcdiTile<TI, SDF, UPD, TYV>, S::TX * (S::TY + 1), acdi_blocks<TI>()>(L, k_acdi_tile<TI, SDF, UPD, TYV>,
                                              tile::grid_of<TYV>(g, kz),
                                              dim3(S::TX, S::TY + 1), acdi_smem<TI, SDF, TYV>(), g, sc, kz, u, v, w, nx,
                                              ny, nz, phi, psi, hist, fx, fy, fz, psi_out, L.wrap);
