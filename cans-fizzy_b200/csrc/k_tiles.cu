@@ -102,16 +102,20 @@ struct YoungsTile {
       }
       cp_commit();
     };
-    // vertex plane kk+1/2 from cell planes kk and kk+1
-    auto vertices = [&](int kk) {
+    // the thread's first vertex, and (vertex warp) its second: place in the
+    // cell plane of its (-x,-y) cell
+    const int q2 = tid - NT + NTT;
+    const int vs1 = tid % VX + PX * (tid / VX), vs2 = q2 % VX + PX * (q2 / VX);
+    const bool second = tid >= NT && q2 < VXY;
+    // vertex plane kk+1/2, into ring slot sv, from cell planes kk and kk+1
+    auto vertices = [&](int kk, int sv) {
       const T* lo = pl[kk % NCP];
       const T* hi = pl[(kk + 1) % NCP];
-      T* ox = vn[(kk + NVP) % NVP][0];
-      T* oy = vn[(kk + NVP) % NVP][1];
-      T* oz = vn[(kk + NVP) % NVP][2];
+      T* ox = vn[sv][0];
+      T* oy = vn[sv][1];
+      T* oz = vn[sv][2];
       const T d1 = (T)g.dxi, d2 = (T)g.dyi, dz = (T)g.dzci[kk];
-      auto vertex = [&](int q) {
-        const int a = q % VX, b = q / VX, s = a + PX * b;
+      auto vertex = [&](int q, int s) {
         const T ccc = lo[s], pcc = lo[s + 1], cpc = lo[s + PX], ppc = lo[s + PX + 1];
         const T ccp = hi[s], pcp = hi[s + 1], cpp = hi[s + PX], ppp = hi[s + PX + 1];
         const T mx = T(0.25) * ((pcc + ppc + pcp + ppp) - (ccc + cpc + ccp + cpp)) * d1;
@@ -122,8 +126,8 @@ struct YoungsTile {
         oy[q] = my * inv;
         oz[q] = mz * inv;
       };
-      vertex(tid);  // tid < NTT <= VXY
-      if (tid >= NT && tid - NT + NTT < VXY) vertex(tid - NT + NTT);
+      vertex(tid, vs1);  // tid < NTT <= VXY
+      if (second) vertex(q2, vs2);
     };
 
     issue(kb - 1);
@@ -132,8 +136,9 @@ struct YoungsTile {
     issue(kb + 2);
     cp_wait<1>();
     __syncthreads();  // planes kb-1, kb, kb+1 are in
-    vertices(kb - 1);
-    vertices(kb);
+    int v0 = 0, v1 = 1, v2 = 2;  // slots of vertex planes k-1/2, k+1/2 and k+3/2
+    vertices(kb - 1, v0);
+    vertices(kb, v1);
     __syncthreads();  // plane kb-1's slot is refilled at the first level
 
     const int i = i0 + tx, j = j0 + ty;
@@ -148,10 +153,10 @@ struct YoungsTile {
       __syncthreads();  // plane k+2 is in; vertex planes k-1/2 and k+1/2 are complete
       // one pass: vertex plane k+3/2 (for level k+1) and the cells of level k,
       // which read the other two vertex planes
-      if (k + 1 <= ke) vertices(k + 1);
+      if (k + 1 <= ke) vertices(k + 1, v2);
       if (act) {
-        const T* lo = vn[(k - 1 + NVP) % NVP][0];
-        const T* hi = vn[k % NVP][0];
+        const T* lo = vn[v0][0];
+        const T* hi = vn[v1][0];
         const int vm = tx + VX * ty;  // the (-x,-y) vertex of the cell
         // vertex q: 0 (+,+,+) 1 (+,-,+) 2 (+,+,-) 3 (+,-,-) 4 (-,+,+) 5 (-,-,+) 6 (-,+,-) 7 (-,-,-)
         const int off[8] = {VX + 1, 1, VX + 1, 1, VX, 0, VX, 0};
@@ -186,6 +191,10 @@ struct YoungsTile {
           kappa[h] = kap;
         });
       }
+      const int vk = v0;
+      v0 = v1;
+      v1 = v2;
+      v2 = vk;
     }
   }
 };

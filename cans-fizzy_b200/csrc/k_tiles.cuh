@@ -48,29 +48,32 @@ __device__ __forceinline__ bool plane_cell(const Geo& g, int i0, int j0, int kk,
   return ii <= g.nx + 1 && jj <= g.ny + 1;
 }
 
-// The elements of a plane that one of NTH threads copies (at most two), placed
-// once instead of at every level: element q at halo index off + kk*sxy, or
-// nothing (a zero) outside the array.  With the
-// ring slots rotated instead of reduced modulo 3, at 256^3: ACDI tile 527 -> 516 us
-// (FP32 383 -> 371), Youngs 272 -> 252 us (FP32 220 -> 193): both issue about 70%
-// of the slots, over a third of them integer arithmetic.
+// The elements of a plane that one of NTH threads copies, placed once instead of
+// at every level: element q at halo index off + kk*sxy, or nothing (a zero)
+// outside the array.  With the ring slots rotated instead of reduced modulo 3, at
+// 256^3: ACDI tile 527 -> 516 us (FP32 383 -> 371), Youngs 272 -> 247 us (FP32 220
+// -> 192): both issue about 70% of the slots, over a third of them integer
+// arithmetic.
 template <int PX, int PXY, int NTH>
 struct PlaneCopy {
-  static_assert(NTH < PXY && PXY <= 2 * NTH, "two elements per thread");
-  int q0, off0, off1;
-  bool ok0, ok1, two;
+  static constexpr int NE = (PXY + NTH - 1) / NTH;
+  int q0, off[NE];
+  bool ok[NE];
   __device__ __forceinline__ PlaneCopy(const Geo& g, int i0, int j0, int tid) : q0(tid) {
-    two = tid + NTH < PXY;
-    ok0 = plane_cell<PX>(g, i0, j0, 0, tid, &off0);
-    ok1 = plane_cell<PX>(g, i0, j0, 0, two ? tid + NTH : tid, &off1);
-    const int in = g.h(i0 - 1, j0 - 1, 0);  // an address of the array for what is not read
-    if (!ok0) off0 = in;
-    if (!ok1) off1 = in;
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const int q = tid + e * NTH;
+      ok[e] = plane_cell<PX>(g, i0, j0, 0, q < PXY ? q : tid, &off[e]);
+      if (!ok[e]) off[e] = g.h(i0 - 1, j0 - 1, 0);  // an address of the array for what is not read
+    }
   }
   template <typename F>
   __device__ __forceinline__ void each(int plane, F f) const {
-    f(q0, off0 + plane, ok0);
-    if (two) f(q0 + NTH, off1 + plane, ok1);
+#pragma unroll
+    for (int e = 0; e < NE; ++e) {
+      const int q = q0 + e * NTH;
+      if ((e + 1) * NTH <= PXY || q < PXY) f(q, off[e] + plane, ok[e]);
+    }
   }
 };
 
