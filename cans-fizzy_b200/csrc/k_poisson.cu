@@ -1719,7 +1719,7 @@ struct ZSolvePart {
     T* tile = reinterpret_cast<T*>(smraw);        // [nz][NC]
     T* red = tile + (size_t)nz * NC;               // [2P][4][NC]: sub, diag, sup, rhs of the reduced rows
     T* xb = red + (size_t)8 * P * NC;              // [2P][NC]: x_s, x_e of every chunk
-    const bool serial0 = zsing && __ldg(lam) == 0.;
+    const bool serial0 = __ldg(lam) == 0.;  // singular, or (one Dirichlet wall) the worst conditioned column
     if (bk.x == 0) {  // the extra block, first: its chain is the longest (as the last one: 94 -> 101 us at 256^3)
       if (serial0) zsolve_serial0<T>(ncol, nz, a, b, c, piv0, df0, work, zsing, tile);
       return;
