@@ -43,6 +43,14 @@ __device__ __forceinline__ Blk blk_here() {
 // follows that wait, so at most one kernel waits behind another.  Both are
 // no-ops in a plain launch, but not free: kernels of a point per thread in
 // blocks of 128 keep blk_here (fillps at 256^3 took 137 instead of 93 us).
+// The kernel's lifetime then overlaps that of a kernel which still writes what
+// it reads after the wait, and a load through the read-only path (__ldg, or a
+// pointer both const and __restrict__) is only defined for data that nothing
+// writes meanwhile: in these kernels fields and step scalars are read by plain
+// loads, through pointers without __restrict__ (the outputs keep theirs, which
+// is what tells the compiler that inputs and outputs differ); only a plan's
+// tables (twiddles, lam, a, b, c, elimination factors) are read that way, all
+// of them complete before any kernel that reads them starts.
 __device__ __forceinline__ Blk blk_chain() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

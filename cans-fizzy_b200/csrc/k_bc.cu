@@ -87,7 +87,7 @@ __device__ __forceinline__ void bc_stage_point(const Geo& g, const BcField& F, E
 template <int STAGE>
 struct BcStage {
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const BcGroup& grp,
-      const DevScalars* __restrict__ sc) {
+      const DevScalars* sc) {
     if (sc != nullptr && sc->halted) return;
     const int fi = bk.y;
     if (fi >= grp.nf) return;
@@ -98,7 +98,7 @@ struct BcStage {
   }
 };
 template <int STAGE>
-__global__ void k_bc_stage(Geo g, BcGroup grp, const DevScalars* __restrict__ sc) {
+__global__ void k_bc_stage(Geo g, BcGroup grp, const DevScalars* sc) {
   BcStage<STAGE>::run(blk_chain(), g, grp, sc);
 }
 
@@ -157,7 +157,7 @@ __device__ __forceinline__ E bc_apply(const BcStep& s, E v) {
 // ghost planes, or those and the face plane n
 struct BcAll {
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const BcGroup& grp,
-      const DevScalars* __restrict__ sc, int px, int py, int pz) {
+      const DevScalars* sc, int px, int py, int pz) {
     if (sc != nullptr && sc->halted) return;
     const BcField& F = grp.f[bk.y];
     const int NX = g.nx + 2, NY = g.ny + 2, NZ = g.nz + 2;
@@ -184,7 +184,7 @@ struct BcAll {
     else put(static_cast<double*>(F.p));
   }
 };
-__global__ void k_bc_all(Geo g, BcGroup grp, const DevScalars* __restrict__ sc, int px, int py, int pz) {
+__global__ void k_bc_all(Geo g, BcGroup grp, const DevScalars* sc, int px, int py, int pz) {
   BcAll::run(blk_chain(), g, grp, sc, px, py, pz);
 }
 

@@ -79,10 +79,10 @@ constexpr int kMomSlots = 48;
 template <typename TI, int TYV, int OPT, int STG>
 struct MomentumTile {
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const Phys& ph,
-      const DevScalars* __restrict__ sc, int kz, const double* __restrict__ u, const double* __restrict__ v,
-      const double* __restrict__ w, const double* __restrict__ psi, const double* __restrict__ psio,
-      const TI* __restrict__ fx, const TI* __restrict__ fy, const TI* __restrict__ fz, const double* __restrict__ p,
-      const double* __restrict__ po, const TI* __restrict__ kappa, const double* __restrict__ s,
+      const DevScalars* sc, int kz, const double* u, const double* v,
+      const double* w, const double* psi, const double* psio,
+      const TI* fx, const TI* fy, const TI* fz, const double* p,
+      const double* po, const TI* kappa, const double* s,
       const SurfSplit& sp, TI* __restrict__ duo, TI* __restrict__ dvo, TI* __restrict__ dwo, double* __restrict__ uo,
       double* __restrict__ vo, double* __restrict__ wo, const HaloMaps& maps, int wrap) {
     constexpr bool BUOY = (OPT & kMomBuoy) != 0, BAL = (OPT & kMomBal) != 0;
@@ -208,22 +208,22 @@ struct MomentumTile {
     double p_c = 0., po_c = 0., pso_c = 0., k_c = 0.;
     if (act) {
       const int cm = g.h(i, j, kb - 1);
-      u_ccm = (T)__ldg(u + cm);
-      v_ccm = (T)__ldg(v + cm);
-      w_ccm = (T)__ldg(w + cm);
-      w_pcm = (T)__ldg(w + cm + 1);
-      w_cpm = (T)__ldg(w + cm + sx);
-      c_ccm = (T)__ldg(psi + cm);
-      c_pcm = (T)__ldg(psi + cm + 1);
-      c_cpm = (T)__ldg(psi + cm + sx);
-      flx_z_ccm = rho * w_ccm + drho * __ldg(fz + cm);
-      flx_z_pcm = rho * w_pcm + drho * __ldg(fz + cm + 1);
-      flx_z_cpm = rho * w_cpm + drho * __ldg(fz + cm + sx);
+      u_ccm = (T)u[cm];
+      v_ccm = (T)v[cm];
+      w_ccm = (T)w[cm];
+      w_pcm = (T)w[cm + 1];
+      w_cpm = (T)w[cm + sx];
+      c_ccm = (T)psi[cm];
+      c_pcm = (T)psi[cm + 1];
+      c_cpm = (T)psi[cm + sx];
+      flx_z_ccm = rho * w_ccm + drho * fz[cm];
+      flx_z_pcm = rho * w_pcm + drho * fz[cm + 1];
+      flx_z_cpm = rho * w_cpm + drho * fz[cm + sx];
       const int c0 = cm + sxy;
-      p_c = __ldg(p + c0);
-      po_c = __ldg(po + c0);
-      pso_c = __ldg(psio + c0);
-      k_c = (double)__ldg(kappa + c0);
+      p_c = p[c0];
+      po_c = po[c0];
+      pso_c = psio[c0];
+      k_c = (double)kappa[c0];
     }
 
     issue(kb);
@@ -283,11 +283,11 @@ struct MomentumTile {
             asm volatile("prefetch.global.L2 [%0];" ::"l"(po + c2));
             asm volatile("prefetch.global.L2 [%0];" ::"l"(kappa + c2));
           }
-          pso_x = __ldg(psio + c + 1); pso_y = __ldg(psio + c + sx); pso_z = __ldg(psio + c + sxy);
-          p_x = __ldg(p + c + 1); p_y = __ldg(p + c + sx); p_z = __ldg(p + c + sxy);
-          po_x = __ldg(po + c + 1); po_y = __ldg(po + c + sx); po_z = __ldg(po + c + sxy);
-          k_x = (double)__ldg(kappa + c + 1); k_y = (double)__ldg(kappa + c + sx);
-          k_z = (double)__ldg(kappa + c + sxy);
+          pso_x = psio[c + 1]; pso_y = psio[c + sx]; pso_z = psio[c + sxy];
+          p_x = p[c + 1]; p_y = p[c + sx]; p_z = p[c + sxy];
+          po_x = po[c + 1]; po_y = po[c + sx]; po_z = po[c + sxy];
+          k_x = (double)kappa[c + 1]; k_y = (double)kappa[c + sx];
+          k_z = (double)kappa[c + sxy];
         }
         const double hu0 = first ? 0. : (double)duo[t], hv0 = first ? 0. : (double)dvo[t],
                      hw0 = first ? 0. : (double)dwo[t];
@@ -447,7 +447,7 @@ struct MomentumTile {
         sdv = sdv - (dpdy_e + rhoyp * ph.irho0 * (dpy - dpdy_e));
         sdw = sdw - (dpdz_e + rhozp * ph.irho0 * (dpz - dpdz_e));
         if (BUOY) {
-          const double s_c = __ldg(s + c), s_x = __ldg(s + c + 1), s_y = __ldg(s + c + sx), s_z = __ldg(s + c + sxy);
+          const double s_c = s[c], s_x = s[c + 1], s_y = s[c + sx], s_z = s[c + sxy];
           const double factorxp = ph.rhobeta + ph.drhobeta * psixp;
           const double factoryp = ph.rhobeta + ph.drhobeta * psiyp;
           const double factorzp = ph.rhobeta + ph.drhobeta * psizp;
@@ -495,10 +495,10 @@ struct MomentumTile {
 };
 template <typename TI, int TYV, int OPT, int STG>
 __global__ void __launch_bounds__(tile::Shape<TYV>::NT, 512 / tile::Shape<TYV>::NT) k_momentum_tile(Geo g, Phys ph,
-    const DevScalars* __restrict__ sc, int kz, const double* __restrict__ u, const double* __restrict__ v,
-    const double* __restrict__ w, const double* __restrict__ psi, const double* __restrict__ psio,
-    const TI* __restrict__ fx, const TI* __restrict__ fy, const TI* __restrict__ fz, const double* __restrict__ p,
-    const double* __restrict__ po, const TI* __restrict__ kappa, const double* __restrict__ s, const SurfSplit sp,
+    const DevScalars* sc, int kz, const double* u, const double* v,
+    const double* w, const double* psi, const double* psio,
+    const TI* fx, const TI* fy, const TI* fz, const double* p,
+    const double* po, const TI* kappa, const double* s, const SurfSplit sp,
     TI* __restrict__ duo, TI* __restrict__ dvo, TI* __restrict__ dwo, double* __restrict__ uo,
     double* __restrict__ vo, double* __restrict__ wo, const __grid_constant__ HaloMaps maps, int wrap) {
   MomentumTile<TI, TYV, OPT, STG>::run(blk_chain(), g, ph, sc, kz, u, v, w, psi, psio, fx, fy, fz, p, po, kappa, s, sp,

@@ -346,8 +346,8 @@ constexpr int kXLinesMax = 16;
 template <typename T, bool FUSED, int MC, int LC>
 struct FftXFwd {
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
-      const DevScalars* __restrict__ sc, const double* __restrict__ src, const double* __restrict__ u,
-      const double* __restrict__ v, const double* __restrict__ w, const Phys& ph, T* __restrict__ work, int Lrt) {
+      const DevScalars* sc, const double* src, const double* u,
+      const double* v, const double* w, const Phys& ph, T* __restrict__ work, int Lrt) {
     if (HALTED(sc)) return;
     extern __shared__ __align__(16) unsigned char smraw[];
     T* sm = reinterpret_cast<T*>(smraw);
@@ -375,10 +375,10 @@ struct FftXFwd {
       if (cb >= 0) {
         const int c = cb + i + 1;
         if (FUSED) {
-          x = ph.rho0 * ((__ldg(w + c) - __ldg(w + c - g.sxy)) * ldz[line] +
-                         (__ldg(v + c) - __ldg(v + c - g.sx)) * dtidyi + (__ldg(u + c) - __ldg(u + c - 1)) * dtidxi);
+          x = ph.rho0 * ((w[c] - w[c - g.sxy]) * ldz[line] +
+                         (v[c] - v[c - g.sx]) * dtidyi + (u[c] - u[c - 1]) * dtidxi);
         } else {
-          x = __ldg(src + c);
+          x = src[c];
         }
       }
       return x;
@@ -413,9 +413,9 @@ struct FftXFwd {
   }
 };
 template <typename T, bool FUSED, int MC, int LC>
-__global__ void __launch_bounds__(256) k_fft_x_fwd(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
-    const double* __restrict__ src, const double* __restrict__ u, const double* __restrict__ v,
-    const double* __restrict__ w, Phys ph, T* __restrict__ work, int Lrt) {
+__global__ void __launch_bounds__(256) k_fft_x_fwd(Geo g, LinePlan pl, const DevScalars* sc,
+    const double* src, const double* u, const double* v,
+    const double* w, Phys ph, T* __restrict__ work, int Lrt) {
   FftXFwd<T, FUSED, MC, LC>::run(blk_chain(), g, pl, sc, src, u, v, w, ph, work, Lrt);
 }
 
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(256) k_fft_x_fwd(Geo g, LinePlan pl, const Dev
 template <typename T, bool ADD, int MC, int LC>
 struct FftXBwd {
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
-      const DevScalars* __restrict__ sc, const T* __restrict__ work, double normfft, double* __restrict__ dst,
+      const DevScalars* sc, const T* work, double normfft, double* __restrict__ dst,
       int Lrt, int wrap) {
     if (HALTED(sc)) return;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -482,8 +482,8 @@ struct FftXBwd {
   }
 };
 template <typename T, bool ADD, int MC, int LC>
-__global__ void __launch_bounds__(256) k_fft_x_bwd(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
-    const T* __restrict__ work, double normfft, double* __restrict__ dst, int Lrt, int wrap) {
+__global__ void __launch_bounds__(256) k_fft_x_bwd(Geo g, LinePlan pl, const DevScalars* sc,
+    const T* work, double normfft, double* __restrict__ dst, int Lrt, int wrap) {
   FftXBwd<T, ADD, MC, LC>::run(blk_chain(), g, pl, sc, work, normfft, dst, Lrt, wrap);
 }
 
@@ -574,8 +574,8 @@ __device__ __forceinline__ cx<T> real_fwd_Xc(const LinePlan& pl, cx<T> zk, cx<T>
 template <typename T, bool FUSED, int R>
 struct FftXFwdW {
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
-      const DevScalars* __restrict__ sc, const double* __restrict__ src, const double* __restrict__ u,
-      const double* __restrict__ v, const double* __restrict__ w, const Phys& ph, T* __restrict__ work) {
+      const DevScalars* sc, const double* src, const double* u,
+      const double* v, const double* w, const Phys& ph, T* __restrict__ work) {
     if (HALTED(sc)) return;
     constexpr int M = 32 * R, N = 2 * M;
     __shared__ cx<T> sz[8][M];
@@ -591,9 +591,9 @@ struct FftXFwdW {
       const double dzk = FUSED ? dti * g.dzfi[kk] : 0.;
       auto get = [&](int c) -> double {
         if (FUSED)
-          return ph.rho0 * ((__ldg(w + c) - __ldg(w + c - g.sxy)) * dzk + (__ldg(v + c) - __ldg(v + c - g.sx)) * dtidyi +
-                            (__ldg(u + c) - __ldg(u + c - 1)) * dtidxi);
-        return __ldg(src + c);
+          return ph.rho0 * ((w[c] - w[c - g.sxy]) * dzk + (v[c] - v[c - g.sx]) * dtidyi +
+                            (u[c] - u[c - 1]) * dtidxi);
+        return src[c];
       };
       cx<T> z[R];
 #pragma unroll
@@ -622,16 +622,16 @@ struct FftXFwdW {
   }
 };
 template <typename T, bool FUSED, int R>
-__global__ void __launch_bounds__(256) k_fft_x_fwd_w(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
-    const double* __restrict__ src, const double* __restrict__ u, const double* __restrict__ v,
-    const double* __restrict__ w, Phys ph, T* __restrict__ work) {
+__global__ void __launch_bounds__(256) k_fft_x_fwd_w(Geo g, LinePlan pl, const DevScalars* sc,
+    const double* src, const double* u, const double* v,
+    const double* w, Phys ph, T* __restrict__ work) {
   FftXFwdW<T, FUSED, R>::run(blk_chain(), g, pl, sc, src, u, v, w, ph, work);
 }
 
 template <typename T, bool ADD, int R>
 struct FftXBwdW {
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
-      const DevScalars* __restrict__ sc, const T* __restrict__ work, double normfft, double* __restrict__ dst,
+      const DevScalars* sc, const T* work, double normfft, double* __restrict__ dst,
       int wrap) {
     if (HALTED(sc)) return;
     constexpr int M = 32 * R, N = 2 * M;
@@ -693,8 +693,8 @@ struct FftXBwdW {
   }
 };
 template <typename T, bool ADD, int R>
-__global__ void __launch_bounds__(256) k_fft_x_bwd_w(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
-    const T* __restrict__ work, double normfft, double* __restrict__ dst, int wrap) {
+__global__ void __launch_bounds__(256) k_fft_x_bwd_w(Geo g, LinePlan pl, const DevScalars* sc,
+    const T* work, double normfft, double* __restrict__ dst, int wrap) {
   FftXBwdW<T, ADD, R>::run(blk_chain(), g, pl, sc, work, normfft, dst, wrap);
 }
 
@@ -705,7 +705,7 @@ __global__ void __launch_bounds__(256) k_fft_x_bwd_w(Geo g, LinePlan pl, const D
 template <typename T, int DIR, int MC, int LC>
 struct FftY {
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
-      const DevScalars* __restrict__ sc, T* __restrict__ work, int Lrt) {
+      const DevScalars* sc, T* __restrict__ work, int Lrt) {
     if (HALTED(sc)) return;
     extern __shared__ __align__(16) unsigned char smraw[];
     T* sm = reinterpret_cast<T*>(smraw);
@@ -755,7 +755,7 @@ struct FftY {
   }
 };
 template <typename T, int DIR, int MC, int LC>
-__global__ void __launch_bounds__(256) k_fft_y(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
+__global__ void __launch_bounds__(256) k_fft_y(Geo g, LinePlan pl, const DevScalars* sc,
                                                T* __restrict__ work, int Lrt) {
   FftY<T, DIR, MC, LC>::run(blk_chain(), g, pl, sc, work, Lrt);
 }
@@ -821,7 +821,7 @@ struct FftY2 {
   static constexpr int A = Y2Shape<MC>::A, B = Y2Shape<MC>::B, L = Y2Shape<MC>::L, NT = B * L;
   static_assert(A % 2 == 0 && A / 2 <= B, "the pair pass fits in the B-pass threads");
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
-      const DevScalars* __restrict__ sc, T* __restrict__ work) {
+      const DevScalars* sc, T* __restrict__ work) {
     if (HALTED(sc)) return;
     constexpr int M = MC;
     __shared__ cx<T> sb[M * L];  // [k1][j2][line]
@@ -955,8 +955,8 @@ struct FftX2Fwd {
   static constexpr int A = Y2Shape<MC>::A, B = Y2Shape<MC>::B, L = Y2Shape<MC>::L, NT = B * L, P = B + 1;
   static constexpr int LP = A * P + (B == 4 ? 4 : 0);  // line pitch: two lines per quarter warp when B = 4
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
-      const DevScalars* __restrict__ sc, const double* __restrict__ src, const double* __restrict__ u,
-      const double* __restrict__ v, const double* __restrict__ w, const Phys& ph, T* __restrict__ work) {
+      const DevScalars* sc, const double* src, const double* u,
+      const double* v, const double* w, const Phys& ph, T* __restrict__ work) {
     if (HALTED(sc)) return;
     constexpr int M = MC, N = 2 * MC;
     __shared__ cx<T> sb[L * LP];  // [line][k1][j2]
@@ -969,9 +969,9 @@ struct FftX2Fwd {
     const double dtidxi = dti * g.dxi, dtidyi = dti * g.dyi, dzk = FUSED ? dti * g.dzfi[kk] : 0.;
     auto get = [&](int c) -> double {
       if (FUSED)
-        return ph.rho0 * ((__ldg(w + c) - __ldg(w + c - g.sxy)) * dzk + (__ldg(v + c) - __ldg(v + c - g.sx)) * dtidyi +
-                          (__ldg(u + c) - __ldg(u + c - 1)) * dtidxi);
-      return __ldg(src + c);
+        return ph.rho0 * ((w[c] - w[c - g.sxy]) * dzk + (v[c] - v[c - g.sx]) * dtidyi +
+                          (u[c] - u[c - 1]) * dtidxi);
+      return src[c];
     };
     cx<T>* sl = sb + l * LP;
     {  // A-point DFTs over j1, j2 = q
@@ -1018,8 +1018,8 @@ struct FftX2Fwd {
 };
 template <typename T, bool FUSED, int MC>
 __global__ void __launch_bounds__(FftX2Fwd<T, FUSED, MC>::NT, 3) k_fft_x2_fwd(Geo g, LinePlan pl,
-    const DevScalars* __restrict__ sc, const double* __restrict__ src, const double* __restrict__ u,
-    const double* __restrict__ v, const double* __restrict__ w, Phys ph, T* __restrict__ work) {
+    const DevScalars* sc, const double* src, const double* u,
+    const double* v, const double* w, Phys ph, T* __restrict__ work) {
   FftX2Fwd<T, FUSED, MC>::run(blk_chain(), g, pl, sc, src, u, v, w, ph, work);
 }
 
@@ -1028,7 +1028,7 @@ struct FftX2Bwd {
   static constexpr int A = Y2Shape<MC>::A, B = Y2Shape<MC>::B, L = Y2Shape<MC>::L, NT = B * L, P = B + 1;
   static constexpr int LP = A * P + (B == 4 ? 4 : 0);
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
-      const DevScalars* __restrict__ sc, const T* __restrict__ work, double normfft, double* __restrict__ dst,
+      const DevScalars* sc, const T* work, double normfft, double* __restrict__ dst,
       int wrap) {
     if (HALTED(sc)) return;
     constexpr int N = 2 * MC;
@@ -1108,14 +1108,14 @@ struct FftX2Bwd {
 };
 template <typename T, bool ADD, int MC>
 __global__ void __launch_bounds__(FftX2Bwd<T, ADD, MC>::NT, 4) k_fft_x2_bwd(Geo g, LinePlan pl,
-    const DevScalars* __restrict__ sc, const T* __restrict__ work, double normfft, double* __restrict__ dst,
+    const DevScalars* sc, const T* work, double normfft, double* __restrict__ dst,
     int wrap) {
   FftX2Bwd<T, ADD, MC>::run(blk_chain(), g, pl, sc, work, normfft, dst, wrap);
 }
 
 template <typename T, int DIR, int MC>
 __global__ void __launch_bounds__(FftY2<T, DIR, MC>::NT, 3) k_fft_y2(Geo g, LinePlan pl,
-                                                                   const DevScalars* __restrict__ sc,
+                                                                   const DevScalars* sc,
                                                                    T* __restrict__ work) {
   FftY2<T, DIR, MC>::run(blk_chain(), g, pl, sc, work);
 }
@@ -1140,7 +1140,7 @@ template <typename T, int DIR>
 struct FftYW {
   static constexpr int NT = kW * kW;
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
-      const DevScalars* __restrict__ sc, T* __restrict__ work) {
+      const DevScalars* sc, T* __restrict__ work) {
     if (HALTED(sc)) return;
     constexpr int M = kW * kW;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -1229,7 +1229,7 @@ struct FftYW {
 };
 template <typename T, int DIR>
 __global__ void __launch_bounds__(FftYW<T, DIR>::NT, 2) k_fft_y512(Geo g, LinePlan pl,
-                                                                  const DevScalars* __restrict__ sc,
+                                                                  const DevScalars* sc,
                                                                   T* __restrict__ work) {
   FftYW<T, DIR>::run(blk_chain(), g, pl, sc, work);
 }
@@ -1240,8 +1240,8 @@ template <typename T, bool FUSED>
 struct FftXWFwd {
   static constexpr int NT = kW * kW, P = kW + 1;
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
-      const DevScalars* __restrict__ sc, const double* __restrict__ src, const double* __restrict__ u,
-      const double* __restrict__ v, const double* __restrict__ w, const Phys& ph, T* __restrict__ work) {
+      const DevScalars* sc, const double* src, const double* u,
+      const double* v, const double* w, const Phys& ph, T* __restrict__ work) {
     if (HALTED(sc)) return;
     constexpr int M = kW * kW, N = 2 * M;
     extern __shared__ __align__(16) unsigned char smraw[];
@@ -1255,9 +1255,9 @@ struct FftXWFwd {
     const double dtidxi = dti * g.dxi, dtidyi = dti * g.dyi, dzk = FUSED ? dti * g.dzfi[kk] : 0.;
     auto get = [&](int c) -> double {
       if (FUSED)
-        return ph.rho0 * ((__ldg(w + c) - __ldg(w + c - g.sxy)) * dzk + (__ldg(v + c) - __ldg(v + c - g.sx)) * dtidyi +
-                          (__ldg(u + c) - __ldg(u + c - 1)) * dtidxi);
-      return __ldg(src + c);
+        return ph.rho0 * ((w[c] - w[c - g.sxy]) * dzk + (v[c] - v[c - g.sx]) * dtidyi +
+                          (u[c] - u[c - 1]) * dtidxi);
+      return src[c];
     };
     {
       cx<T> z[kW], y[kW];
@@ -1289,9 +1289,9 @@ struct FftXWFwd {
   }
 };
 template <typename T, bool FUSED>
-__global__ void __launch_bounds__(256, 2) k_fft_x512_fwd(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
-    const double* __restrict__ src, const double* __restrict__ u, const double* __restrict__ v,
-    const double* __restrict__ w, Phys ph, T* __restrict__ work) {
+__global__ void __launch_bounds__(256, 2) k_fft_x512_fwd(Geo g, LinePlan pl, const DevScalars* sc,
+    const double* src, const double* u, const double* v,
+    const double* w, Phys ph, T* __restrict__ work) {
   FftXWFwd<T, FUSED>::run(blk_chain(), g, pl, sc, src, u, v, w, ph, work);
 }
 
@@ -1299,7 +1299,7 @@ template <typename T, bool ADD>
 struct FftXWBwd {
   static constexpr int NT = kW * kW, P = kW + 1;
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const LinePlan& pl,
-      const DevScalars* __restrict__ sc, const T* __restrict__ work, double normfft, double* __restrict__ dst,
+      const DevScalars* sc, const T* work, double normfft, double* __restrict__ dst,
       int wrap) {
     if (HALTED(sc)) return;
     constexpr int N = 2 * kW * kW;
@@ -1353,8 +1353,8 @@ struct FftXWBwd {
   }
 };
 template <typename T, bool ADD>
-__global__ void __launch_bounds__(256, 2) k_fft_x512_bwd(Geo g, LinePlan pl, const DevScalars* __restrict__ sc,
-    const T* __restrict__ work, double normfft, double* __restrict__ dst, int wrap) {
+__global__ void __launch_bounds__(256, 2) k_fft_x512_bwd(Geo g, LinePlan pl, const DevScalars* sc,
+    const T* work, double normfft, double* __restrict__ dst, int wrap) {
   FftXWBwd<T, ADD>::run(blk_chain(), g, pl, sc, work, normfft, dst, wrap);
 }
 
@@ -1567,7 +1567,7 @@ __device__ void thomas_factored(int n, const double* __restrict__ a, const T* __
 template <typename T>
 struct ZSolveF {
   static __device__ __forceinline__ void run(const Blk& bk, int ncol, int nz, const double* __restrict__ a,
-      const T* __restrict__ piv, const T* __restrict__ df, const DevScalars* __restrict__ sc,
+      const T* __restrict__ piv, const T* __restrict__ df, const DevScalars* sc,
       T* __restrict__ work) {
     if (HALTED(sc)) return;
     const int col = bk.x * blockDim.x + threadIdx.x;
@@ -1577,7 +1577,7 @@ struct ZSolveF {
 };
 template <typename T>
 __global__ void __launch_bounds__(128) k_zsolve_f(int ncol, int nz, const double* __restrict__ a,
-    const T* __restrict__ piv, const T* __restrict__ df, const DevScalars* __restrict__ sc, T* __restrict__ work) {
+    const T* __restrict__ piv, const T* __restrict__ df, const DevScalars* sc, T* __restrict__ work) {
   ZSolveF<T>::run(blk_chain(), ncol, nz, a, piv, df, sc, work);
 }
 
@@ -1585,7 +1585,7 @@ template <typename T>
 struct ZSolve {
   static __device__ __forceinline__ void run(const Blk& bk, int ncol, int nz, const double* __restrict__ lam,
       const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
-      const DevScalars* __restrict__ sc, T* __restrict__ work, int zsing) {
+      const DevScalars* sc, T* __restrict__ work, int zsing) {
     if (HALTED(sc)) return;
     extern __shared__ __align__(16) unsigned char smraw[];
     T* dchk = reinterpret_cast<T*>(smraw);  // [nch][blockDim]
@@ -1599,7 +1599,7 @@ struct ZSolve {
 template <typename T>
 __global__ void __launch_bounds__(128) k_zsolve(int ncol, int nz, const double* __restrict__ lam,
     const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
-    const DevScalars* __restrict__ sc, T* __restrict__ work, int zsing) {
+    const DevScalars* sc, T* __restrict__ work, int zsing) {
   ZSolve<T>::run(blk_chain(), ncol, nz, lam, a, b, c, sc, work, zsing);
 }
 
@@ -1710,7 +1710,7 @@ template <typename T, int CH, int P, bool EXACT>
 struct ZSolvePart {
   static __device__ __forceinline__ void run(const Blk& bk, int ncol, int nz, const double* __restrict__ lam,
       const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
-      const T* __restrict__ piv0, const T* __restrict__ df0, const DevScalars* __restrict__ sc,
+      const T* __restrict__ piv0, const T* __restrict__ df0, const DevScalars* sc,
       T* __restrict__ work, int zsing) {
     if (HALTED(sc)) return;
     static_assert(CH >= 3, "a chunk needs an interior row");
@@ -1837,7 +1837,7 @@ template <typename T, int CH, int P, bool EXACT>
 __global__ void __launch_bounds__(32 * P, P == 8 ? (sizeof(T) == 4 ? 4 : 2) : 1) k_zsolve_part(int ncol, int nz,
     const double* __restrict__ lam, const double* __restrict__ a, const double* __restrict__ b,
     const double* __restrict__ c, const T* __restrict__ piv0, const T* __restrict__ df0,
-    const DevScalars* __restrict__ sc, T* __restrict__ work, int zsing) {
+    const DevScalars* sc, T* __restrict__ work, int zsing) {
   ZSolvePart<T, CH, P, EXACT>::run(blk_chain(), ncol, nz, lam, a, b, c, piv0, df0, sc, work, zsing);
 }
 
@@ -1846,7 +1846,7 @@ template <typename T>
 struct ZSolvePeriodic {
   static __device__ __forceinline__ void run(const Blk& bk, int ncol, int nz, const double* __restrict__ lam,
       const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
-      const DevScalars* __restrict__ sc, T* __restrict__ work, T* __restrict__ work2) {
+      const DevScalars* sc, T* __restrict__ work, T* __restrict__ work2) {
     if (HALTED(sc)) return;
     extern __shared__ __align__(16) unsigned char smraw[];
     T* dchk = reinterpret_cast<T*>(smraw);
@@ -1876,7 +1876,7 @@ struct ZSolvePeriodic {
 template <typename T>
 __global__ void __launch_bounds__(128) k_zsolve_periodic(int ncol, int nz, const double* __restrict__ lam,
     const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
-    const DevScalars* __restrict__ sc, T* __restrict__ work, T* __restrict__ work2) {
+    const DevScalars* sc, T* __restrict__ work, T* __restrict__ work2) {
   ZSolvePeriodic<T>::run(blk_chain(), ncol, nz, lam, a, b, c, sc, work, work2);
 }
 
@@ -1885,7 +1885,7 @@ template <typename T>
 struct ZSolvePeriodicF {
   static __device__ __forceinline__ void run(const Blk& bk, int ncol, int nz, const double* __restrict__ lam,
       const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
-      const T* __restrict__ piv, const T* __restrict__ df, const DevScalars* __restrict__ sc,
+      const T* __restrict__ piv, const T* __restrict__ df, const DevScalars* sc,
       T* __restrict__ work, T* __restrict__ work2) {
     if (HALTED(sc)) return;
     const int col = bk.x * blockDim.x + threadIdx.x;
@@ -1912,7 +1912,7 @@ struct ZSolvePeriodicF {
 template <typename T>
 __global__ void __launch_bounds__(128) k_zsolve_periodic_f(int ncol, int nz, const double* __restrict__ lam,
     const double* __restrict__ a, const double* __restrict__ b, const double* __restrict__ c,
-    const T* __restrict__ piv, const T* __restrict__ df, const DevScalars* __restrict__ sc, T* __restrict__ work,
+    const T* __restrict__ piv, const T* __restrict__ df, const DevScalars* sc, T* __restrict__ work,
     T* __restrict__ work2) {
   ZSolvePeriodicF<T>::run(blk_chain(), ncol, nz, lam, a, b, c, piv, df, sc, work, work2);
 }

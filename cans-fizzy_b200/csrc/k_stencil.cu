@@ -178,8 +178,8 @@ void launch_thinc_transport(const Launch& L, const Geo& g, const DevScalars* sc,
 constexpr int kPhiPer = 4;  // points per thread of k_cmpt_phi
 template <bool ACDI, typename TO>
 struct CmptPhi {
-  static __device__ __forceinline__ void run(const Blk& bk, int n, const DevScalars* __restrict__ sc,
-      const double* __restrict__ psi, TO* __restrict__ phi) {
+  static __device__ __forceinline__ void run(const Blk& bk, int n, const DevScalars* sc,
+      const double* psi, TO* __restrict__ phi) {
     if (HALTED(sc)) return;
     // kPhiPer points per thread, a block's points contiguous: loads first
     const int q0 = bk.x * blockDim.x * kPhiPer + threadIdx.x;
@@ -187,7 +187,7 @@ struct CmptPhi {
 #pragma unroll
     for (int m = 0; m < kPhiPer; ++m) {
       const int q = q0 + m * blockDim.x;
-      ps[m] = q < n ? LD(psi, q) : 0.;
+      ps[m] = q < n ? psi[q] : 0.;
     }
 #pragma unroll
     for (int m = 0; m < kPhiPer; ++m) {
@@ -203,7 +203,7 @@ struct CmptPhi {
   }
 };
 template <bool ACDI, typename TO>
-__global__ void k_cmpt_phi(int n, const DevScalars* __restrict__ sc, const double* __restrict__ psi,
+__global__ void k_cmpt_phi(int n, const DevScalars* sc, const double* psi,
                            TO* __restrict__ phi) {
   CmptPhi<ACDI, TO>::run(blk_chain(), n, sc, psi, phi);
 }
@@ -792,8 +792,8 @@ struct CorrecUpdatep {
   // all loads first (p at level k+1 is the next level's own p), then the
   // updates, so that a warp has many independent loads in flight
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const Phys& ph,
-      const DevScalars* __restrict__ sc, const double* __restrict__ p, double* __restrict__ u,
-      double* __restrict__ v, double* __restrict__ w, const double* __restrict__ pp, double* __restrict__ pout,
+      const DevScalars* sc, const double* p, double* __restrict__ u,
+      double* __restrict__ v, double* __restrict__ w, const double* pp, double* __restrict__ pout,
       int wrap) {
     constexpr int KC = kCorrecLevels;
     if (HALTED(sc)) return;
@@ -810,16 +810,16 @@ struct CorrecUpdatep {
     for (int q = 0; q < KC; ++q) {
       const int k = k0 + q, c = c0 + q * g.sxy;
       if (k <= g.nz + 1) {
-        pc[q] = LD(p, c);
-        px[q] = xin ? LD(p, c + 1) : 0.;
-        py[q] = yin ? LD(p, c + g.sx) : 0.;
+        pc[q] = p[c];
+        px[q] = xin ? p[c + 1] : 0.;
+        py[q] = yin ? p[c + g.sx] : 0.;
         uo[q] = xin ? u[c] : 0.;
         vo[q] = yin ? v[c] : 0.;
         wo[q] = k <= g.nz ? w[c] : 0.;
-        pq[q] = (ij_p && k_p(k)) ? LD(pp, c) : 0.;
+        pq[q] = (ij_p && k_p(k)) ? pp[c] : 0.;
       }
     }
-    pc[KC] = (k0 + KC - 1 <= g.nz) ? LD(p, c0 + KC * g.sxy) : 0.;
+    pc[KC] = (k0 + KC - 1 <= g.nz) ? p[c0 + KC * g.sxy] : 0.;
 #pragma unroll
     for (int q = 0; q < KC; ++q) {
       const int k = k0 + q, c = c0 + q * g.sxy;
@@ -846,10 +846,10 @@ struct CorrecUpdatep {
     }
   }
 };
-__global__ void __launch_bounds__(256) k_correc_updatep(Geo g, Phys ph, const DevScalars* __restrict__ sc,
-                                                        const double* __restrict__ p, double* __restrict__ u,
+__global__ void __launch_bounds__(256) k_correc_updatep(Geo g, Phys ph, const DevScalars* sc,
+                                                        const double* p, double* __restrict__ u,
                                                         double* __restrict__ v, double* __restrict__ w,
-                                                        const double* __restrict__ pp, double* __restrict__ pout,
+                                                        const double* pp, double* __restrict__ pout,
                                                         int wrap) {
   CorrecUpdatep::run(blk_chain(), g, ph, sc, p, u, v, w, pp, pout, wrap);
 }
@@ -993,7 +993,7 @@ __global__ void k_gamma_max(Geo g, DevScalars* __restrict__ sc, double* __restri
   if (threadIdx.x == 0) part[blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)] = vel;
 }
 // maximum of n non-negative partials, one block
-__device__ __forceinline__ double reduce_max_partials(int n, const double* __restrict__ part) {
+__device__ __forceinline__ double reduce_max_partials(int n, const double* part) {
   double m = 0.;
   for (int q = threadIdx.x; q < n; q += blockDim.x) m = fmax(m, part[q]);
   return block_max(m);
@@ -1018,21 +1018,21 @@ void launch_gamma(const Launch& L, const Geo& g, const Phys& ph, DevScalars* sc,
 }
 
 // the per-point maximum of chkdt (src/chkdt.f90:47-78)
-__device__ __forceinline__ double chkdt_cell(const Geo& g, int i, int j, int k, const double* __restrict__ u,
-                                             const double* __restrict__ v, const double* __restrict__ w) {
+__device__ __forceinline__ double chkdt_cell(const Geo& g, int i, int j, int k, const double* u,
+                                             const double* v, const double* w) {
   const int c = g.h(i, j, k), sx = g.sx, sxy = g.sxy;
   const double dxi = recip_rn(g.dx), dyi = recip_rn(g.dy);
-  const double ux = fabs(LD(u, c));
-  const double vx = 0.25 * fabs(LD(v, c) + LD(v, c - sx) + LD(v, c + 1) + LD(v, c + 1 - sx));
-  const double wx = 0.25 * fabs(LD(w, c) + LD(w, c - sxy) + LD(w, c + 1) + LD(w, c + 1 - sxy));
+  const double ux = fabs(u[c]);
+  const double vx = 0.25 * fabs(v[c] + v[c - sx] + v[c + 1] + v[c + 1 - sx]);
+  const double wx = 0.25 * fabs(w[c] + w[c - sxy] + w[c + 1] + w[c + 1 - sxy]);
   const double dtix = ux * dxi + vx * dyi + wx * g.dzfi[k];
-  const double uy = 0.25 * fabs(LD(u, c) + LD(u, c + sx) + LD(u, c - 1 + sx) + LD(u, c - 1));
-  const double vy = fabs(LD(v, c));
-  const double wy = 0.25 * fabs(LD(w, c) + LD(w, c + sx) + LD(w, c + sx - sxy) + LD(w, c - sxy));
+  const double uy = 0.25 * fabs(u[c] + u[c + sx] + u[c - 1 + sx] + u[c - 1]);
+  const double vy = fabs(v[c]);
+  const double wy = 0.25 * fabs(w[c] + w[c + sx] + w[c + sx - sxy] + w[c - sxy]);
   const double dtiy = uy * dxi + vy * dyi + wy * g.dzfi[k];
-  const double uz = 0.25 * fabs(LD(u, c) + LD(u, c - 1) + LD(u, c - 1 + sxy) + LD(u, c + sxy));
-  const double vz = 0.25 * fabs(LD(v, c) + LD(v, c - sx) + LD(v, c - sx + sxy) + LD(v, c + sxy));
-  const double wz = fabs(LD(w, c));
+  const double uz = 0.25 * fabs(u[c] + u[c - 1] + u[c - 1 + sxy] + u[c + sxy]);
+  const double vz = 0.25 * fabs(v[c] + v[c - sx] + v[c - sx + sxy] + v[c + sxy]);
+  const double wz = fabs(w[c]);
   const double dtiz = uz * dxi + vz * dyi + wz * g.dzci[k];
   return fmax(dtix, fmax(dtiy, dtiz));
 }
@@ -1176,8 +1176,8 @@ void launch_chkdiv(const Launch& L, const Geo& g, DevScalars* sc, double* partia
 constexpr int kReduceThreads = 256;
 struct StepReduce {
   static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, DevScalars* __restrict__ sc, int acdi,
-      double* __restrict__ part, const double* __restrict__ u, const double* __restrict__ v,
-      const double* __restrict__ w) {
+      double* __restrict__ part, const double* u, const double* v,
+      const double* w) {
     if (HALTED(sc)) return;
     const bool chk = sc->check_now != 0;
     if (!acdi && !chk) return;
@@ -1194,12 +1194,12 @@ struct StepReduce {
             const int r = r0 + q * bk.nx;
             if (r < nrows) {
               const int c = g.h(i, r % g.ny + 1, r / g.ny + 1);
-              u0[q] = LD(u, c);
-              u1[q] = LD(u, c - 1);
-              v0[q] = LD(v, c);
-              v1[q] = LD(v, c - g.sx);
-              w0[q] = LD(w, c);
-              w1[q] = LD(w, c - g.sxy);
+              u0[q] = u[c];
+              u1[q] = u[c - 1];
+              v0[q] = v[c];
+              v1[q] = v[c - g.sx];
+              w0[q] = w[c];
+              w1[q] = w[c - g.sxy];
             }
           }
 #pragma unroll
@@ -1218,14 +1218,14 @@ struct StepReduce {
         for (int i = threadIdx.x + 1; i <= g.nx; i += blockDim.x) {
           const int c = g.h(i, j, k);
           if (acdi) {
-            const double uc = 0.5 * (LD(u, c) + LD(u, c - 1));
-            const double vc = 0.5 * (LD(v, c) + LD(v, c - g.sx));
-            const double wc = 0.5 * (LD(w, c) + LD(w, c - g.sxy));
+            const double uc = 0.5 * (u[c] + u[c - 1]);
+            const double vc = 0.5 * (v[c] + v[c - g.sx]);
+            const double wc = 0.5 * (w[c] + w[c - g.sxy]);
             velmax = fmax(velmax, vel2(uc, vc, wc));
           }
           dtimax = fmax(dtimax, chkdt_cell(g, i, j, k, u, v, w));
-          const double div = (LD(w, c) - LD(w, c - g.sxy)) * g.dzfi[k] + (LD(v, c) - LD(v, c - g.sx)) * g.dyi +
-                             (LD(u, c) - LD(u, c - 1)) * g.dxi;
+          const double div = (w[c] - w[c - g.sxy]) * g.dzfi[k] + (v[c] - v[c - g.sx]) * g.dyi +
+                             (u[c] - u[c - 1]) * g.dxi;
           divsum += div;
           divmax = fmax(divmax, fabs(div));
         }
@@ -1246,14 +1246,14 @@ struct StepReduce {
 };
 __global__ void __launch_bounds__(kReduceThreads) k_step_reduce(Geo g, DevScalars* __restrict__ sc, int acdi,
                                                                 double* __restrict__ part,
-                                                                const double* __restrict__ u,
-                                                                const double* __restrict__ v,
-                                                                const double* __restrict__ w) {
+                                                                const double* u,
+                                                                const double* v,
+                                                                const double* w) {
   StepReduce::run(blk_chain(), g, sc, acdi, part, u, v, w);
 }
 struct StepReduceFinal {
   static __device__ __forceinline__ void run(const Blk& bk, const Phys& ph, DevScalars* __restrict__ sc, int nb,
-      const double* __restrict__ part) {
+      const double* part) {
     if (HALTED(sc)) return;
     const bool chk = sc->check_now != 0;
     if (!ph.acdi && !chk) return;
@@ -1272,7 +1272,7 @@ struct StepReduceFinal {
     }
   }
 };
-__global__ void k_step_reduce_final(Phys ph, DevScalars* __restrict__ sc, int nb, const double* __restrict__ part) {
+__global__ void k_step_reduce_final(Phys ph, DevScalars* __restrict__ sc, int nb, const double* part) {
   StepReduceFinal::run(blk_chain(), ph, sc, nb, part);
 }
 void launch_step_reductions(const Launch& L, const Geo& g, const Phys& ph, DevScalars* sc, double* partial,

@@ -69,8 +69,8 @@ __device__ __forceinline__ T inv_norm_eps(T s) {
 // ---------------------------------------------------------------------------
 template <typename TI, int TYV>
 struct YoungsTile {
-  static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const DevScalars* __restrict__ sc, int kz,
-      const TI* __restrict__ phi, TI* __restrict__ normx, TI* __restrict__ normy, TI* __restrict__ normz,
+  static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const DevScalars* sc, int kz,
+      const TI* phi, TI* __restrict__ normx, TI* __restrict__ normy, TI* __restrict__ normz,
       TI* __restrict__ kappa, int wrap) {
     using namespace tile;
     using SH = Shape<TYV>;
@@ -199,8 +199,8 @@ struct YoungsTile {
   }
 };
 template <typename TI, int TYV>
-__global__ void __launch_bounds__(tile::Shape<TYV>::NT + tile::Shape<TYV>::TX, 4) k_youngs_tile(Geo g, const DevScalars* __restrict__ sc, int kz,
-                                                          const TI* __restrict__ phi, TI* __restrict__ normx,
+__global__ void __launch_bounds__(tile::Shape<TYV>::NT + tile::Shape<TYV>::TX, 4) k_youngs_tile(Geo g, const DevScalars* sc, int kz,
+                                                          const TI* phi, TI* __restrict__ normx,
                                                           TI* __restrict__ normy, TI* __restrict__ normz,
                                                           TI* __restrict__ kappa, int wrap) {
   YoungsTile<TI, TYV>::run(blk_chain(), g, sc, kz, phi, normx, normy, normz, kappa, wrap);
@@ -253,10 +253,10 @@ constexpr size_t acdi_smem() {
 // and d on exit.  Without UPD, dpsidt receives d.
 template <typename TI, bool SDF, bool UPD, int TYV>
 struct AcdiTile {
-  static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const DevScalars* __restrict__ sc, int kz,
-      const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ w,
-      const TI* __restrict__ nx_, const TI* __restrict__ ny_, const TI* __restrict__ nz_,
-      const TI* __restrict__ phi, const double* __restrict__ psi, TI* __restrict__ dpsidt, TI* __restrict__ fx,
+  static __device__ __forceinline__ void run(const Blk& bk, const Geo& g, const DevScalars* sc, int kz,
+      const double* u, const double* v, const double* w,
+      const TI* nx_, const TI* ny_, const TI* nz_,
+      const TI* phi, const double* psi, TI* __restrict__ dpsidt, TI* __restrict__ fx,
       TI* __restrict__ fy, TI* __restrict__ fz, double* __restrict__ psi_out, int wrap) {
     using namespace tile;
     using SH = Shape<TYV>;
@@ -320,14 +320,14 @@ struct AcdiTile {
     __syncthreads();
     T up_zm = T(0), rg_zm = T(0);
     if (act)
-      face(2, (T)g.dzci[kb - 1], s2, qc, s0, qc, (T)__ldg(w + g.h(i, j, kb - 1)), &up_zm,
+      face(2, (T)g.dzci[kb - 1], s2, qc, s0, qc, (T)w[g.h(i, j, kb - 1)], &up_zm,
            &rg_zm);
     __syncthreads();  // plane kb-1's slot is refilled next
 
     T vx_n = T(0), vy_n = T(0), vz_n = T(0);
     if (act) {
       const int c = g.h(i, j, kb);
-      vx_n = (T)__ldg(u + c); vy_n = (T)__ldg(v + c); vz_n = (T)__ldg(w + c);
+      vx_n = (T)u[c]; vy_n = (T)v[c]; vz_n = (T)w[c];
     }
     for (int k = kb; k <= ke; ++k) {
       if (k + 2 <= ke + 1) issue(k + 2, s2);
@@ -342,7 +342,7 @@ struct AcdiTile {
         const int c = g.h(i, j, k);
         const T vx = vx_n, vy = vy_n, vz = vz_n;
         if (k < ke) {
-          vx_n = (T)__ldg(u + c + g.sxy); vy_n = (T)__ldg(v + c + g.sxy); vz_n = (T)__ldg(w + c + g.sxy);
+          vx_n = (T)u[c + g.sxy]; vy_n = (T)v[c + g.sxy]; vz_n = (T)w[c + g.sxy];
         }
         if (UPD && !first2) dO_pre = dpsidt[g.t(i, j, k)];
         T upx, rgx, upy, rgy;
@@ -363,13 +363,13 @@ struct AcdiTile {
           if (e < TY) {
             if (j0 + e <= g.ny) {
               const int q = PX * (e + 1), f = e * (TX + 1);
-              face(0, dxi, s0, q, s0, q + 1, (T)__ldg(u + g.h(i0 - 1, j0 + e, k)), &f_up[f], &f_rg[f]);
+              face(0, dxi, s0, q, s0, q + 1, (T)u[g.h(i0 - 1, j0 + e, k)], &f_up[f], &f_rg[f]);
             }
           } else {
             const int a = e - TY;
             if (i0 + a <= g.nx) {
               const int q = a + 1, f = NFX + a;
-              face(1, dyi, s0, q, s0, q + PX, (T)__ldg(v + g.h(i0 + a, j0 - 1, k)), &f_up[f], &f_rg[f]);
+              face(1, dyi, s0, q, s0, q + PX, (T)v[g.h(i0 + a, j0 - 1, k)], &f_up[f], &f_rg[f]);
             }
           }
         }
@@ -416,10 +416,10 @@ struct AcdiTile {
 template <typename TI>
 constexpr int acdi_blocks() { return sizeof(TI) == 8 ? 3 : 4; }
 template <typename TI, bool SDF, bool UPD, int TYV>
-__global__ void __launch_bounds__(tile::Shape<TYV>::TX * (tile::Shape<TYV>::TY + 1), acdi_blocks<TI>()) k_acdi_tile(Geo g, const DevScalars* __restrict__ sc, int kz,
-    const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ w,
-    const TI* __restrict__ nx_, const TI* __restrict__ ny_, const TI* __restrict__ nz_,
-    const TI* __restrict__ phi, const double* __restrict__ psi, TI* __restrict__ dpsidt,
+__global__ void __launch_bounds__(tile::Shape<TYV>::TX * (tile::Shape<TYV>::TY + 1), acdi_blocks<TI>()) k_acdi_tile(Geo g, const DevScalars* sc, int kz,
+    const double* u, const double* v, const double* w,
+    const TI* nx_, const TI* ny_, const TI* nz_,
+    const TI* phi, const double* psi, TI* __restrict__ dpsidt,
     TI* __restrict__ fx, TI* __restrict__ fy, TI* __restrict__ fz, double* __restrict__ psi_out, int wrap) {
   AcdiTile<TI, SDF, UPD, TYV>::run(blk_chain(), g, sc, kz, u, v, w, nx_, ny_, nz_, phi, psi, dpsidt, fx, fy, fz,
       psi_out, wrap);
