@@ -19,6 +19,7 @@
 #pragma once
 
 #include <cstring>
+#include <mutex>
 #include <type_traits>
 #include <utility>
 #include <vector>
@@ -117,11 +118,28 @@ struct Recorder {
   std::vector<RecEntry> e;
 };
 
+// Raise kernel `k`'s limit of dynamic shared memory on the current device to
+// `smem` bytes; it is never lowered, since one instance serves launches of
+// different sizes (the partitioned z solve: columns of 200 and of 250 levels).
+// The lock keeps another thread's larger limit from being overwritten between
+// the look at it and the change.
+inline std::mutex& smem_limit_lock() {
+  static std::mutex m;
+  return m;
+}
+template <class K>
+int raise_smem_limit(K k, size_t smem) {
+  if (smem <= 48 * 1024) return 0;
+  std::lock_guard<std::mutex> hold(smem_limit_lock());
+  cudaFuncAttributes at;
+  if (cudaFuncGetAttributes(&at, k) != cudaSuccess) return 1;
+  if ((size_t)at.maxDynamicSharedSizeBytes >= smem) return 0;
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess ? 0 : 1;
+}
+
 template <class F, int NT, int MINB, class P>
 int batch_prepare(const RecEntry& e) {
-  if (e.smem <= 48 * 1024) return 0;
-  return cudaFuncSetAttribute(k_batch<F, NT, MINB, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)e.smem) == cudaSuccess ? 0 : 1;
+  return raise_smem_limit(k_batch<F, NT, MINB, P>, e.smem);
 }
 
 template <class F, int NT, int MINB, class P>

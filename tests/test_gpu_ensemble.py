@@ -105,3 +105,45 @@ def test_batched_two_pass_line_transforms():
         for nm in ("u", "v", "w", "p", "psi"):
             assert np.array_equal(a.get(nm), b.get(nm)), nm
     ens.close()
+
+
+def test_groups_that_share_a_kernel_with_unequal_shared_memory():
+    """Two batched groups whose columns of 250 and 200 levels run the same
+    instance of the partitioned z solve (chunks of at most 32 levels) with
+    83 and 70 KB of shared memory: the second group's launch must not lower
+    the limit that the first one's needs."""
+    specs = [W._bubble_case(16, 2, nz, 1.0, 2.0 / 16, nz / 16.0, 100.0, 10.0, sigma, 0.4, True)
+             for nz, sigma in ((250, 5.0), (250, 8.0), (200, 5.0), (200, 8.0))]
+    single = _build(specs)
+    for c in single:
+        assert c.step(6) == 0
+    batch = _build(specs)
+    ens = C.Ensemble(batch, batch=2)
+    rc, _ = ens.step(6)
+    assert rc == 0
+    assert ens.groups() == (2, 4)
+    for a, b in zip(single, batch):
+        for nm in ("u", "v", "w", "p", "psi"):
+            assert np.array_equal(a.get(nm), b.get(nm)), nm
+    ens.close()
+
+
+@pytest.mark.parametrize("batching", [1, 2])
+def test_ensemble_of_much_work(batching):
+    """Above 8 million cells the tile kernels' blocks take 32 levels instead
+    of 8: 9.0 million in five cases, two of them in one group."""
+    specs = [W._bubble_case(n, n, 2 * n, 1.0, 1.0, 2.0, r, 10.0, 5.0, 0.4, False)
+             for n, r in ((128, 10.0), (96, 10.0), (96, 100.0), (64, 10.0), (64, 100.0))]
+    specs.append(W._bubble_case(40, 36, 70, 1.0, 0.9, 1.75, 10.0, 10.0, 5.0, 0.4, False))
+    assert sum(p.ng[0] * p.ng[1] * p.ng[2] for p, _ in specs) > 8e6
+    single = _build(specs)
+    for c in single:
+        assert c.step(3) == 0
+    batch = _build(specs)
+    ens = C.Ensemble(batch, batch=batching)
+    rc, _ = ens.step(3)
+    assert rc == 0
+    for a, b in zip(single, batch):
+        for nm in ("u", "v", "w", "p", "psi"):
+            assert np.array_equal(a.get(nm), b.get(nm)), nm
+    ens.close()
