@@ -340,7 +340,7 @@ int alloc_f32_solver(cansfz_ctx* c) {
     launch_z_factors(c->L, c->g, c->pl, true, c->g.nx * c->g.ny, c->pl.zpivf, c->pl.zdff);
     CK(cudaGetLastError());
   }
-  if (!c->pl.zpiv0f && z_part_ok(c->g, c->pl)) {
+  if (!c->pl.zpiv0f && c->pl.zsing && z_part_ok(c->g, c->pl)) {
     const size_t n = (size_t)c->n[2];
     if ((rc = dalloc(c, &c->pl.zpiv0f, n)) || (rc = dalloc(c, &c->pl.zdf0f, n))) return rc;
     launch_z_factors(c->L, c->g, c->pl, true, 1, c->pl.zpiv0f, c->pl.zdf0f);
@@ -494,7 +494,7 @@ int setup_solver(cansfz_ctx* c) {
     launch_z_factors(c->L, c->g, c->pl, false, nx * ny, c->pl.zpiv, c->pl.zdf);
     CK(cudaGetLastError());
   }
-  if (z_part_ok(c->g, c->pl)) {
+  if (c->pl.zsing && z_part_ok(c->g, c->pl)) {
     if ((rc = dalloc(c, &c->pl.zpiv0, (size_t)nz)) || (rc = dalloc(c, &c->pl.zdf0, (size_t)nz))) return rc;
     launch_z_factors(c->L, c->g, c->pl, false, 1, c->pl.zpiv0, c->pl.zdf0);
     CK(cudaGetLastError());

@@ -1626,14 +1626,30 @@ __global__ void __launch_bounds__(128) k_zsolve(int ncol, int nz, const double* 
 // blocks per SM at nz = 256), with few the length of the chain of dependent
 // steps, CH + 2P + 2P + 2CH against the column sweep's 2 nz (a whole step at 64x64x128: 203 -> 184 us, at 64x2x128: 138 -> 126 us, the solve itself 28 -> 9 us).
 //
-// The order of elimination differs from gaussel's (src/solver.f90:151-177)
-// only by round-off for these diagonally dominant systems (|b + lambda| >=
-// |a| + |c|).  The one singular system, the (0,0) mode of an all-periodic/
-// Neumann problem, whose eps-shifted pivot (src/solver.f90:163-167) fixes
-// the solution's constant, is solved by one more block in gaussel's own
-// order (thomas_column's operations, the factors read where the plan has
-// them); the tile of column 0 leaves that column's result to it (what its
-// lane reads there meanwhile, right-hand side or solution, goes nowhere).
+// Pivots without cancellation.  b + lambda - a*d, gaussel's pivot
+// (src/solver.f90:151-177), is the difference of nearly equal numbers where
+// the row sum is small, |lambda| dz^2 << 1: the lowest modes lose about
+// (2 nz/pi)^2 roundings, in whatever order the rows are eliminated.  Here a
+// row is known by its off-diagonals and its sum E = a + b + c + lambda instead
+// of its diagonal (Grassmann, Taksar and Heyman's form of elimination for
+// diagonally dominant M-matrices).  Eliminating its neighbour gives the row
+// off-diagonals and a sum that are again sums of terms of one sign, and the
+// pivot is E less the off-diagonals, of one sign too.  Relative error of a
+// random right-hand side's solution (the 200 lowest columns and 200 others, in
+// the 2-norm against 113-bit arithmetic): gaussel's order, these chunks with
+// pivots by differences, and this form:
+//   256^3 Neumann walls          2.1e-13  2.3e-13  4.1e-16   FP32 1.4e-4  1.2e-4  2.2e-7
+//   512x256x256 stretched (1.5)  2.7e-13  3.4e-13  4.4e-16   FP32 7.2e-5  7.1e-5  2.4e-7
+//   128^3                        3.7e-15  6.3e-15  2.9e-16   FP32 1.9e-5  1.8e-5  1.3e-7
+//   512x8x24, cubic cells        1.2e-12  9.8e-13  3.6e-16   FP32 3.3e-4  4.2e-4  1.9e-7
+// Two more operations per row and sweep, one load fewer: 92.9 -> 91.6 us at
+// 256^3, FP32 64.2 -> 60.4 us; 14.6 -> 16.0 us at 128^3.
+// The one singular system, the (0,0) mode of an all-periodic/Neumann
+// problem, whose eps-shifted pivot (src/solver.f90:163-167) fixes the
+// solution's constant, is solved by one more block in gaussel's own order
+// (thomas_column's operations, the factors read where the plan has them); the
+// tile of column 0 leaves that column's result to it (what its lane reads
+// there meanwhile, right-hand side or solution, goes nowhere).
 // ---------------------------------------------------------------------------
 constexpr int ZP_NC = 32;  // columns per tile
 // the chunk lengths built (a chunk of fewer levels runs in the next longer one)
@@ -1652,7 +1668,7 @@ __device__ __forceinline__ void cp16_cg(void* sdst, const void* gsrc) {
 
 template <typename T>
 constexpr size_t zpart_smem(int nz, int P) {
-  return sizeof(T) * ((size_t)nz * ZP_NC + (size_t)8 * P * ZP_NC + (size_t)2 * P * ZP_NC);
+  return sizeof(T) * ((size_t)nz * ZP_NC + (size_t)8 * P * ZP_NC + (size_t)2 * P * ZP_NC + nz);
 }
 
 // the singular column: gaussel's elimination order and rounding, by one thread
@@ -1717,14 +1733,15 @@ struct ZSolvePart {
     constexpr int NC = ZP_NC;
     extern __shared__ __align__(16) unsigned char smraw[];
     T* tile = reinterpret_cast<T*>(smraw);        // [nz][NC]
-    T* red = tile + (size_t)nz * NC;               // [2P][4][NC]: sub, diag, sup, rhs of the reduced rows
+    T* red = tile + (size_t)nz * NC;               // [2P][4][NC]: sub, row sum, sup, rhs of the reduced rows
     T* xb = red + (size_t)8 * P * NC;              // [2P][NC]: x_s, x_e of every chunk
-    const bool serial0 = __ldg(lam) == 0.;  // singular, or (one Dirichlet wall) the worst conditioned column
-    if (bk.x == 0) {  // the extra block, first: its chain is the longest (as the last one: 94 -> 101 us at 256^3)
+    T* sum = xb + (size_t)2 * P * NC;              // [nz]: the rows' sums a + b + c
+    const bool serial0 = zsing && __ldg(lam) == 0.;
+    if (zsing && bk.x == 0) {  // the extra block, first: its chain is the longest (as the last one: 94 -> 101 us at 256^3)
       if (serial0) zsolve_serial0<T>(ncol, nz, a, b, c, piv0, df0, work, zsing, tile);
       return;
     }
-    const int col0 = (bk.x - 1) * NC, cols = EXACT ? NC : min(NC, ncol - col0);
+    const int col0 = (bk.x - (zsing ? 1 : 0)) * NC, cols = EXACT ? NC : min(NC, ncol - col0);
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int base = EXACT ? CH : nz / P, rem = EXACT ? 0 : nz % P;
     const int len = EXACT ? CH : base + (w < rem ? 1 : 0);
@@ -1739,53 +1756,69 @@ struct ZSolvePart {
     }
     asm volatile("cp.async.commit_group;\n" ::);
     const T lm = (T)__ldg(lam + (in ? col0 + lane : 0));
+    // the chunk's row sums (a level per lane), of what b's rounding left of
+    // them too: t + b is exact or, at a Dirichlet wall, not small
+    for (int l = s + lane; l <= e; l += 32) {
+      const double av = l > 0 ? __ldg(a + l) : 0., cv = l < nz - 1 ? __ldg(c + l) : 0.;
+      const double t = av + cv, tc = t - av;
+      sum[l] = (T)((t + __ldg(b + l)) + ((av - (t - tc)) + (cv - tc)));
+    }
     asm volatile("cp.async.wait_group 0;\n" ::);
     __syncwarp();
     // ---- A: the chunk's two reduced rows.  The downward sweep's pivot
     // reciprocals are those of C's forward sweep (same rows, same first
     // pivot), so they are kept for it and C needs no reciprocal.
+    // Downwards x_i = Y + F x_s - (c/pivot) x_{i+1}, and H = row sum/pivot;
+    // the next row's pivot is its row sum - a H, less its c and its a F.
     T rp[CH - 2];
     {
-      T D = 0, Y = 0, F = 0, U = 0, Z = 0, G = 0;
+      T Y = 0, F = 1, H = 0, Z = 0, G = 1, K = 0;
 #pragma unroll
       for (int t = 0; t < CH - 2; ++t) {
         if (!EXACT && t >= len - 2) break;  // the same for the whole warp
         const int id = s + 1 + t, iu = e - 1 - t;
-        const T ad = (T)__ldg(a + id), cd = (T)__ldg(c + id), bd = (T)__ldg(b + id) + lm;
-        const T au = (T)__ldg(a + iu), cu = (T)__ldg(c + iu), bu = (T)__ldg(b + iu) + lm;
+        const T ad = (T)__ldg(a + id), cd = (T)__ldg(c + id);
+        const T au = (T)__ldg(a + iu), cu = (T)__ldg(c + iu);
         const T dd = tile[id * NC + lane], du = tile[iu * NC + lane];
-        const T rd = recip_rn(t == 0 ? bd : bd - ad * D);
+        T Ed = sum[id] + lm, Eu = sum[iu] + lm;
+        if (t > 0) {
+          Ed -= ad * H;
+          Eu -= cu * K;
+        }
+        const T rd = recip_rn((Ed - cd) - (t == 0 ? ad : ad * F));
         rp[t] = rd;
         Y = (t == 0 ? dd : dd - ad * Y) * rd;
         F = (t == 0 ? -ad : -ad * F) * rd;
-        D = cd * rd;
-        const T ru = recip_rn(t == 0 ? bu : bu - cu * U);
+        H = Ed * rd;
+        const T ru = recip_rn((Eu - au) - (t == 0 ? cu : cu * G));
         Z = (t == 0 ? du : du - cu * Z) * ru;
         G = (t == 0 ? -cu : -cu * G) * ru;
-        U = au * ru;
+        K = Eu * ru;
       }
       T* Rs = red + (size_t)(2 * w) * 4 * NC;
       T* Re = Rs + 4 * NC;
-      const T as = (T)__ldg(a + s), bs = (T)__ldg(b + s) + lm, cs = (T)__ldg(c + s);
-      const T ae = (T)__ldg(a + e), be = (T)__ldg(b + e) + lm, ce = (T)__ldg(c + e);
+      const T as = (T)__ldg(a + s), cs = (T)__ldg(c + s), ae = (T)__ldg(a + e), ce = (T)__ldg(c + e);
       Rs[0 * NC + lane] = w == 0 ? (T)0 : as;
-      Rs[1 * NC + lane] = bs - cs * U;
+      Rs[1 * NC + lane] = (sum[s] + lm) - cs * K;
       Rs[2 * NC + lane] = cs * G;
       Rs[3 * NC + lane] = tile[s * NC + lane] - cs * Z;
       Re[0 * NC + lane] = ae * F;
-      Re[1 * NC + lane] = be - ae * D;
+      Re[1 * NC + lane] = (sum[e] + lm) - ae * H;
       Re[2 * NC + lane] = w == P - 1 ? (T)0 : ce;
       Re[3 * NC + lane] = tile[e * NC + lane] - ae * Y;
     }
     __syncthreads();
-    // ---- B: the reduced system of the 2P chunk-end values
+    // ---- B: the reduced system of the 2P chunk-end values, its pivots from
+    // the row sums too
     if (w == 0) {
-      T Dp = 0, Yp = 0;
+      T Hp = 0, Yp = 0;
       for (int r = 0; r < 2 * P; ++r) {
         T* Rr = red + (size_t)r * 4 * NC;
-        const T sub = Rr[0 * NC + lane], dg = Rr[1 * NC + lane], sup = Rr[2 * NC + lane], rhs = Rr[3 * NC + lane];
-        const T rr = recip_rn(r == 0 ? dg : dg - sub * Dp);
-        Dp = sup * rr;
+        const T sub = Rr[0 * NC + lane], sup = Rr[2 * NC + lane], rhs = Rr[3 * NC + lane];
+        const T E = r == 0 ? Rr[1 * NC + lane] : Rr[1 * NC + lane] - sub * Hp;
+        const T rr = recip_rn(E - sup);
+        Hp = E * rr;
+        const T Dp = sup * rr;
         Yp = (r == 0 ? rhs : rhs - sub * Yp) * rr;
         Rr[0 * NC + lane] = Dp;
         Rr[1 * NC + lane] = Yp;
@@ -2172,8 +2205,9 @@ template <typename T, int CH, int P, bool EXACT>
 static void z_part_go(const Launch& Lc, const Geo& g, const PoissonPlan& pl, const DevScalars* sc) {
   const int ncol = g.nx * g.ny;
   constexpr int MINB = P == 8 ? (sizeof(T) == 4 ? 4 : 2) : 1;
-  // the block of the singular column, and the tiles of columns
-  kgo_chain<ZSolvePart<T, CH, P, EXACT>, 32 * P, MINB>(Lc, k_zsolve_part<T, CH, P, EXACT>, (ncol + ZP_NC - 1) / ZP_NC + 1,
+  // the tiles of columns, and before them the block of the singular column
+  kgo_chain<ZSolvePart<T, CH, P, EXACT>, 32 * P, MINB>(Lc, k_zsolve_part<T, CH, P, EXACT>,
+                                                 (ncol + ZP_NC - 1) / ZP_NC + (pl.zsing ? 1 : 0),
                                                  32 * P, zpart_smem<T>(g.nz, P), ncol, g.nz, pl.lam, pl.a, pl.b, pl.c,
                                                  zpiv0<T>(pl), zdf0<T>(pl), sc, wbuf<T>(pl), pl.zsing);
 }

@@ -1,16 +1,23 @@
-"""The Poisson solve at the edges of its kernels' size ranges, against the
-oracle: the partitioned z solve's chunks (shortest and longest columns,
-columns that the chunks do not divide, a last tile of few columns, FP64 and
-FP32), and the two-pass transforms of 512 points with a partial tile of lines.
+"""The Poisson solve at the edges of its kernels' size ranges: the partitioned
+z solve's chunks (shortest and longest columns, columns that the chunks do not
+divide, a last tile of few columns, FP64 and FP32), thin domains, whose lowest
+modes are the worst conditioned, and the two-pass transforms of 512 points
+with a partial tile of lines.
 
-Bounds: as in test_gpu_parity.test_poisson_bcs, 1e-12 of the largest stored
-value (the constant of the singular mode included) for the FP64 solve.  One
-refinement sweep of the FP32 solve leaves the square of its own relative error:
-up to 7e-4 for a column of 500 levels (2^-24 times a condition number of about
-(2 nz/pi)^2), squared 5e-7, bound 1e-6.  (Not for Neumann walls on a grid whose
-single-precision z quotients make it slightly uneven: there the FP64 residual's
-mean over the singular mode leaves 1e-6 and more whatever the sweeps, in either z solve.)
+The reference is the same discrete system (the eigenvalues and z coefficients
+that the solver holds) solved in extended precision (64-bit significands).
+
+Bounds, relative to the largest value of the solution.  Partitioned columns of
+24 to 512 levels: each of the four transform passes rounds log2(n) <= 9 times,
+a column's solve a few times per chunk: about 50 roundings of 1.1e-16, random in
+sign, and the largest of up to 1e6 values 5 times their deviation: 1e-14.  One
+column per thread (23 and 513 levels): gaussel's order, whose pivots round
+against a condition of (2 nz/pi)^2.  Column 0 of a problem without a Dirichlet
+wall is singular and its constant is fixed by the rounded last pivot in
+gaussel's order, as the oracle's: compared with the oracle apart.
 """
+import math
+
 import numpy as np
 import pytest
 
@@ -20,6 +27,9 @@ from cansfz import case as C
 from test_gpu_parity import _nml
 
 pytestmark = pytest.mark.gpu
+
+EPS = 2.0**-53
+L = np.longdouble
 
 SHAPES = [
     # chunks: 24 levels is the first column the 8 chunks hold, 23 the last they do not
@@ -32,43 +42,159 @@ SHAPES = [
     ("PPPPNN", (512, 6, 9)), ("PPPPDD", (512, 10, 7)), ("NNPPNN", (6, 512, 10)), ("PPPPNN", (20, 512, 3)),
     ("PPPPNN", (512, 512, 4)),
 ]
+# cubic cells, so that lambda*lz^2 of the lowest modes is small
+THIN = [("PPPPNN", (512, 8, 24)), ("PPPPND", (512, 8, 24)), ("PPPPNN", (384, 8, 48)), ("PPPPND", (256, 8, 64)),
+        ("PPPPNN", (128, 32, 100)), ("PPPPDD", (256, 8, 64))]
 
 
-def _system(cbcpre, ng):
-    p = _nml(*ng, cbcpre, l=(1.0, 0.75, 1.2))
+# ---------------------------------------------------------------------------
+# the system in extended precision
+# ---------------------------------------------------------------------------
+def _kind(bc):
+    return {"PP": 0, "NN": 1, "DD": 2}[bc]
+
+
+def _lambda(n, kind, dl):
+    """src/initsolver.f90:81-139, in the order of `_basis`."""
+    if kind == 0:
+        arg = [2.0 * m * math.pi / n for m in range(n // 2 + 1)] + [2.0 * (n - k) * math.pi / n for k in range(1, n // 2)]
+    else:
+        arg = [(m + (kind == 2)) * math.pi / n for m in range(n)]
+    d = 1.0 / dl
+    return np.array([-2.0 * (1.0 - math.cos(a)) * (d * d) for a in arg])
+
+
+def _basis(n, kind):
+    """Orthonormal rows: cosines and sines of a periodic line, the cosines of
+    Neumann walls, the sines of Dirichlet walls."""
+    pi, i = 4 * np.arctan(L(1)), np.arange(n)
+    if kind == 0:
+        k = np.arange(n // 2 + 1)
+        c = np.cos(2 * pi / n * L(1) * ((k[:, None] * i) % n))
+        s = np.sin(2 * pi / n * L(1) * ((k[1:n // 2, None] * i) % n))
+        v = np.concatenate([c, s])
+    else:
+        a = pi / (2 * n) * (((2 * i + 1) * (i[:, None] + (kind == 2))) % (4 * n))
+        v = np.cos(a) if kind == 1 else np.sin(a)
+    return v / np.sqrt((v * v).sum(axis=1, keepdims=True))
+
+
+def _along(v, f, axis):
+    return np.moveaxis(np.tensordot(v, f, axes=(1, axis)), 0, axis)
+
+
+def _exact(p, g, rhs, keep0=True):
+    """The solution of the stored system; keep0: with column 0 (of a problem
+    with a Dirichlet wall), else without it."""
+    bc = [bytes(p.cbcpre[2 * d:2 * d + 2]).decode() for d in range(3)]
+    n = list(p.ng)
+    dl = [p.l[d] / n[d] for d in range(2)]
+    vx, vy = (_basis(n[d], _kind(bc[d])) for d in range(2))
+    lam = _lambda(n[0], _kind(bc[0]), dl[0])[:, None] + _lambda(n[1], _kind(bc[1]), dl[1])
+    dzci, dzfi = g["dzci"], g["dzfi"]
+    a, c = dzfi[1:-1] * dzci[:-2], dzfi[1:-1] * dzci[1:-1]
+    b = -(a + c)
+    b[0] += a[0] * (-1.0 if bc[2][0] == "D" else 1.0)
+    b[-1] += c[-1] * (-1.0 if bc[2][1] == "D" else 1.0)
+    a, b, c, lam = (x.astype(L) for x in (a, b, c, lam))
+    h = _along(vy, _along(vx, rhs.astype(L), 0), 1)
+    if not keep0:
+        h[0, 0] = 0
+        lam[0, 0] = -1
+    d = np.zeros_like(h)
+    d[:, :, 0] = c[0] / (b[0] + lam)
+    h[:, :, 0] /= b[0] + lam
+    for k in range(1, n[2]):
+        z = 1 / (b[k] + lam - a[k] * d[:, :, k - 1])
+        d[:, :, k] = c[k] * z
+        h[:, :, k] = (h[:, :, k] - a[k] * h[:, :, k - 1]) * z
+    for k in range(n[2] - 2, -1, -1):
+        h[:, :, k] -= d[:, :, k] * h[:, :, k + 1]
+    return _along(vx.T, _along(vy.T, h, 1), 0)
+
+
+def _case(cbcpre, ng, thin=False):
+    p = _nml(*ng, cbcpre, l=tuple(n / 512.0 for n in ng) if thin else (1.0, 0.75, 1.2))
     rhs = np.zeros(tuple(n + 2 for n in ng), order="F")
     rhs[1:-1, 1:-1, 1:-1] = np.random.default_rng(5).standard_normal(p.n)
-    if "D" not in cbcpre:
-        rhs[1:-1, 1:-1, 1:-1] -= rhs[1:-1, 1:-1, 1:-1].mean()
     return p, rhs
 
 
-def _compare(a, b, singular):
-    a, b = a[1:-1, 1:-1, 1:-1], b[1:-1, 1:-1, 1:-1]
-    scale = max(np.abs(a).max(), np.abs(b).max())
-    if singular:
-        a, b = a - a.mean(), b - b.mean()
-    return np.abs(a - b).max(), scale, np.abs(b).max()
+def _bound(nz):
+    return 1e-14 if 24 <= nz <= 512 else 4 * EPS * (2 * nz / math.pi) ** 2 + 1e-14
 
 
-@pytest.mark.parametrize("cbcpre,ng", SHAPES)
-def test_solver(cbcpre, ng):
-    p, rhs = _system(cbcpre, ng)
+def _well_posed(cbcpre):
+    return cbcpre if "D" in cbcpre else cbcpre[:5] + "D"
+
+
+# ---------------------------------------------------------------------------
+@pytest.mark.parametrize("cbcpre,ng,thin", [(*s, False) for s in SHAPES] + [(*s, True) for s in THIN])
+def test_solver(cbcpre, ng, thin):
+    """With a Dirichlet wall (the top's where the shape has none): every mode,
+    column 0 included, against the extended-precision solution."""
+    p, rhs = _case(_well_posed(cbcpre), ng, thin)
+    g = C.Case(p)
+    pg = g.field(rhs)
+    g.call("solver", pg)
+    ref = _exact(p, g.grid(), rhs[1:-1, 1:-1, 1:-1])
+    assert np.abs(pg.get()[1:-1, 1:-1, 1:-1] - ref).max() < _bound(ng[2]) * np.abs(ref).max()
+
+
+SINGULAR = [(*s, False) for s in SHAPES if "D" not in s[0]] + [(*s, True) for s in THIN if "D" not in s[0]]
+
+
+@pytest.mark.parametrize("cbcpre,ng,thin", SINGULAR)
+def test_solver_without_a_dirichlet_wall(cbcpre, ng, thin):
+    """Column 0 is each level's sum over x and y, which is exact for whole
+    numbers.  Where the sums are zero, so is column 0's solution, and the
+    others are compared; with 1 added everywhere, which the last pivot blows
+    up, column 0, constant included: a sum of nz equal signs, so nz roundings
+    at most."""
+    p, rhs = _case(cbcpre, ng, thin)
+    inner = rhs[1:-1, 1:-1, 1:-1]
+    inner[:] = np.rint(1024.0 * inner)
+    inner[0, 0] -= inner.sum(axis=(0, 1))
     g, o = C.Case(p), O.Case(p)
     pg = g.field(rhs)
     g.call("solver", pg)
+    ref = _exact(p, g.grid(), inner, keep0=False)
+    assert np.abs(pg.get()[1:-1, 1:-1, 1:-1] - ref).max() < _bound(ng[2]) * np.abs(ref).max()
+    rhs[1:-1, 1:-1, 1:-1] += 1.0
+    pg = g.field(rhs)
+    g.call("solver", pg)
     o.call("solver", rhs)
-    err, scale, _ = _compare(pg.get(), rhs, "D" not in cbcpre)
-    assert err / scale < 1e-12
+    a, b = (f[1:-1, 1:-1, 1:-1].mean(axis=(0, 1)) for f in (pg.get(), rhs))
+    assert np.abs(a - b).max() < 4 * EPS * (ng[2] + 50) * np.abs(b).max()
 
 
-@pytest.mark.parametrize("cbcpre,ng", [("PPPPDD", (12, 10, 24)), ("PPPPDD", (20, 6, 31)), ("PPPPDD", (64, 2, 65)),
-                                       ("PPPPDD", (10, 6, 500)), ("PPPPDD", (512, 6, 9)), ("PPPPNN", (20, 512, 32))])
-def test_solver_refined(cbcpre, ng):
-    p, rhs = _system(cbcpre, ng)
-    g, o = C.Case(p), O.Case(p)
+REFINED = [("PPPPDD", (12, 10, 24), False), ("PPPPDD", (20, 6, 31), False), ("PPPPDD", (64, 2, 65), False),
+           ("PPPPDD", (10, 6, 500), False), ("PPPPDD", (512, 6, 9), False), ("PPPPND", (512, 8, 24), True),
+           ("PPPPND", (256, 8, 64), True), ("PPPPND", (20, 512, 32), False), ("PPPPNN", (20, 512, 32), False),
+           ("PPPPNN", (20, 6, 31), False), ("PPPPNN", (64, 64, 100), False)]
+
+
+@pytest.mark.parametrize("cbcpre,ng,thin", REFINED)
+def test_solver_refined(cbcpre, ng, thin):
+    """The FP32 solve: transforms of 64 to 256 points as split-BF16 GEMMs keep
+    16 bits of a line's largest mode, other lengths 24, and the white right-hand
+    side's smallest modes are 1e-1 of that: 1e-4.  A sweep leaves the same
+    fraction of its residual, in the worst mode ten times that: 1e-3 of the
+    error before, and a second one 1e-3 of that, down to the FP64 rounding.
+    Between Neumann walls, with the sums of each level zero, the pinned column
+    0 is a constant, which is removed."""
+    p, rhs = _case(cbcpre, ng, thin)
+    singular = "D" not in cbcpre
+    inner = rhs[1:-1, 1:-1, 1:-1]
+    if singular:
+        inner[:] = np.rint(1024.0 * inner)
+        inner[0, 0] -= inner.sum(axis=(0, 1))
+    g = C.Case(p)
     rg, pg = g.field(rhs), g.field()
-    g.call("solver_refined", rg, pg, 1)
-    o.call("solver", rhs)
-    err, _, size = _compare(pg.get(), rhs, "D" not in cbcpre)
-    assert err / size < 1e-6
+    ref = _exact(p, g.grid(), inner, keep0=not singular)
+    for sweeps, bound in ((0, 1e-4), (1, 1e-7), (2, 1e-10)):
+        g.call("solver_refined", rg, pg, sweeps)
+        got = pg.get()[1:-1, 1:-1, 1:-1]
+        if singular:
+            got = got - got.mean()
+        assert np.abs(got - ref).max() < bound * np.abs(ref).max(), sweeps
