@@ -298,10 +298,32 @@ bool factorize(int m, int radix[FFT_MAXSTAGES], int* nst) {
   return m == 1 && k <= FFT_MAXSTAGES;
 }
 
-// z solves with fewer columns than this read precomputed elimination factors
-bool zsolve_factored(const cansfz_ctx* c) { return (long long)c->g.nx * c->g.ny < 32768; }
+// The z systems' elimination factors where the column solves read them (once;
+// FP32 ones once the FP32 solver has its buffers): with few columns, where the
+// pivot recurrence's latency bounds the solve -- with many, reading the factors
+// costs more than evaluating them -- and where the partitioned solve, which
+// evaluates its own, does not take the columns.
+int alloc_z_factors(cansfz_ctx* c) {
+  PoissonPlan& pl = c->pl;
+  if ((long long)c->g.nx * c->g.ny >= 32768 || (pl.zmode != 1 && z_part_ok(c->g, pl))) return CANSFZ_OK;
+  const size_t nint = (size_t)c->g.tsize();
+  const int ncol = c->g.nx * c->g.ny;
+  int rc;
+  if (!pl.zdf) {
+    if (!pl.zpiv && (rc = dalloc(c, &pl.zpiv, nint))) return rc;
+    if ((rc = dalloc(c, &pl.zdf, nint))) return rc;
+    launch_z_factors(c->L, c->g, pl, false, ncol, pl.zpiv, pl.zdf);
+    CK(cudaGetLastError());
+  }
+  if (pl.workf && !pl.zdff) {
+    if (!pl.zpivf && (rc = dalloc(c, &pl.zpivf, nint))) return rc;
+    if ((rc = dalloc(c, &pl.zdff, nint))) return rc;
+    launch_z_factors(c->L, c->g, pl, true, ncol, pl.zpivf, pl.zdff);
+    CK(cudaGetLastError());
+  }
+  return CANSFZ_OK;
+}
 
-// FP32 spectral buffers and z factors of the mixed-form solve (once)
 // the split-BF16 matrices of the tensor-core transforms (once), for the
 // line lengths and kinds they serve
 int alloc_xform_gemm(cansfz_ctx* c) {
@@ -329,17 +351,14 @@ int alloc_xform_gemm(cansfz_ctx* c) {
   return CANSFZ_OK;
 }
 
+// FP32 spectral buffers and z factors of the mixed-form solve (once)
 int alloc_f32_solver(cansfz_ctx* c) {
   const size_t nint = (size_t)c->g.tsize();
   int rc;
   if ((rc = alloc_xform_gemm(c))) return rc;
   if (!c->pl.workf && (rc = dalloc(c, &c->pl.workf, nint))) return rc;
   if (c->pl.zper && !c->pl.work2f && (rc = dalloc(c, &c->pl.work2f, nint))) return rc;
-  if (!c->pl.zpivf && zsolve_factored(c)) {
-    if ((rc = dalloc(c, &c->pl.zpivf, nint)) || (rc = dalloc(c, &c->pl.zdff, nint))) return rc;
-    launch_z_factors(c->L, c->g, c->pl, true, c->g.nx * c->g.ny, c->pl.zpivf, c->pl.zdff);
-    CK(cudaGetLastError());
-  }
+  if ((rc = alloc_z_factors(c))) return rc;
   if (!c->pl.zpiv0f && c->pl.zsing && z_part_ok(c->g, c->pl)) {
     const size_t n = (size_t)c->n[2];
     if ((rc = dalloc(c, &c->pl.zpiv0f, n)) || (rc = dalloc(c, &c->pl.zdf0f, n))) return rc;
@@ -485,15 +504,7 @@ int setup_solver(cansfz_ctx* c) {
     rc = dalloc(c, &c->pl.work2, nint);
     if (rc) return rc;
   }
-  // the z systems' elimination factors, once per plan, where the solve has
-  // few columns: there the pivot recurrence's latency bounds the solve,
-  // while with many columns reading the factors costs more than evaluating
-  // them
-  if (zsolve_factored(c)) {
-    if ((rc = dalloc(c, &c->pl.zpiv, nint)) || (rc = dalloc(c, &c->pl.zdf, nint))) return rc;
-    launch_z_factors(c->L, c->g, c->pl, false, nx * ny, c->pl.zpiv, c->pl.zdf);
-    CK(cudaGetLastError());
-  }
+  if ((rc = alloc_z_factors(c))) return rc;
   if (c->pl.zsing && z_part_ok(c->g, c->pl)) {
     if ((rc = dalloc(c, &c->pl.zpiv0, (size_t)nz)) || (rc = dalloc(c, &c->pl.zdf0, (size_t)nz))) return rc;
     launch_z_factors(c->L, c->g, c->pl, false, 1, c->pl.zpiv0, c->pl.zdf0);
@@ -2059,6 +2070,12 @@ int cansfz_set_plan(cansfz_ctx* c, const cansfz_plan* plan) {
     }
   }
   drop_graphs(c);
+  // the column solves' factors; without room for them those solves evaluate
+  // them as they go (the same operations)
+  const int rc = alloc_z_factors(c);
+  if (rc == CANSFZ_ERR_NOMEM) cudaGetLastError();
+  else if (rc) return rc;
+  CK(cudaStreamSynchronize(c->st));
   return CANSFZ_OK;
 }
 

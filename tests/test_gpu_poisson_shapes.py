@@ -198,3 +198,43 @@ def test_solver_refined(cbcpre, ng, thin):
         if singular:
             got = got - got.mean()
         assert np.abs(got - ref).max() < bound * np.abs(ref).max(), sweeps
+
+
+@pytest.mark.parametrize("ng", [(64, 2, 65), (12, 10, 257), (96, 64, 128)])
+def test_column_solve_chosen_later(ng):
+    """zsolve = 1 on a case whose columns the partitioned solve takes: the
+    elimination factors are evaluated when the plan asks for them (FP64, and
+    FP32 where that solver has run or runs later)."""
+    p, rhs = _case("PPPPND", ng)
+    ref = _exact(p, C.Case(p).grid(), rhs[1:-1, 1:-1, 1:-1])
+    for refined_first in (False, True):
+        g = C.Case(p)
+        rg, pg = g.field(rhs), g.field()
+        if refined_first:
+            g.call("solver_refined", rg, pg, 1)
+        q = g.plan()
+        q.zsolve = 1
+        g.set_plan(q)
+        g.call("solver_refined", rg, pg, 1)
+        assert np.abs(pg.get()[1:-1, 1:-1, 1:-1] - ref).max() < 1e-6 * np.abs(ref).max()
+        pg = g.field(rhs)
+        g.call("solver", pg)
+        got = pg.get()[1:-1, 1:-1, 1:-1]
+        assert np.abs(got - ref).max() < (4 * EPS * (2 * ng[2] / math.pi) ** 2 + 1e-14) * np.abs(ref).max()
+
+
+def test_no_factors_where_the_partitioned_solve_takes_the_columns():
+    """Two spectral-size arrays less than a case whose columns are one level
+    too long for it."""
+    import torch
+
+    def used(nz):
+        free = torch.cuda.mem_get_info()[0]
+        case = C.Case(_nml(96, 64, nz))
+        used = free - torch.cuda.mem_get_info()[0]
+        case.close()
+        return used
+
+    used(512)  # the first case loads the module
+    cells = 96 * 64 * 512 * 8
+    assert used(513) - used(512) > 1.5 * cells
