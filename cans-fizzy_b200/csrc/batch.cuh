@@ -181,8 +181,11 @@ inline void kgo(const Launch& L, K k, dim3 grid, dim3 block, size_t smem, V&&...
 // kgo for a kernel that begins with blk_chain
 template <class F, int NT, int MINB, class K, class... V>
 inline void kgo_chain(const Launch& L, K k, dim3 grid, dim3 block, size_t smem, V&&... v) {
-  // Programmatic serialization where this kernel or the one before it has at
-  // most one block per SM.  Between two large kernels it costs more than the
+  // Programmatic serialization where this kernel or the chained one before it has
+  // at most one block per SM.  (Launches by kgo or <<<>>> in between are not
+  // counted: such a kernel has no trigger, so whatever is launched early after
+  // it comes onto the device when its blocks have exited, and there is nothing
+  // to lose.)  Between two large kernels it costs more than the
   // launch gap: the SMs that finish first take more than their share of the
   // waiting blocks (every launch: a step at 160^3 +3%, 90x50x70 +4%; this rule:
   // 64x2x128 -10%, 32^3 -8%, 64^3 -4%, 96^3 -1.6%, 160^3 and 90x50x70 -0.5 and

@@ -189,7 +189,7 @@ struct PoissonPlan {
   double* zdf;
   float* zpivf;
   float* zdff;
-  // the same for column 0 alone (nz values), the singular mode's
+  // the same for column 0 alone (nz values) of a singular problem
   double* zpiv0;
   double* zdf0;
   float* zpiv0f;
@@ -217,8 +217,8 @@ struct Launch {
   // not 0 while an ensemble's step is captured or recorded: the z levels per
   // block of the tile kernels, which there do not split z to fill the GPU
   int batched;
-  // blocks of the context's previous launch (kgo: which launches may come onto
-  // the device early); null: none do
+  // blocks of the context's previous chained launch (kgo_chain: which launches
+  // may come onto the device early); null: none do
   long long* prev_blocks = nullptr;
   // set: launches are recorded for a batched replay instead of issued
   Recorder* rec = nullptr;
@@ -288,7 +288,8 @@ void launch_youngs(const Launch& L, const Geo& g, const DevScalars* sc, const do
 void launch_clip(const Launch& L, const Geo& g, double rmin, double rmax, double* p);
 // the interior of one to three halo-layout fields from as many others; clip:
 // the ghosts of the (one) field are clipped to [0, 1] besides
-void launch_put_interior(const Launch& L, const Geo& g, int nf, const double* const* src, double* const* dst, bool clip);
+void launch_put_interior(const Launch& L, const Geo& g, int nf, const double* const* src, double* const* dst,
+                         bool clip);
 void launch_mom_ad(const Launch& L, const Geo& g, const Phys& ph, const double* fx,
                    const double* fy, const double* fz, const double* u, const double* v,
                    const double* w, const double* psi, double* du, double* dv, double* dw);

@@ -94,7 +94,8 @@ struct cansfz_ctx {
   double *phip = nullptr, *phi = nullptr, *kappa = nullptr, *nx = nullptr, *ny = nullptr, *nz = nullptr;
   double *fx = nullptr, *fy = nullptr, *fz = nullptr;
   double *hpsi = nullptr, *hu = nullptr, *hv = nullptr, *hw = nullptr;       // AB2 histories (interior)
-  double *tu = nullptr, *tv = nullptr, *tw_ = nullptr, *tpsi = nullptr;     // per-procedure scratch (room for a halo field)
+  // per-procedure scratch (room for a halo field)
+  double *tu = nullptr, *tv = nullptr, *tw_ = nullptr, *tpsi = nullptr;
   // scalar (_SCALAR): s by parity like u,v,w,psi; the dsdtrko history (interior)
   double *s[2]{}, *hs = nullptr;
   // balanced capillary split: surf?_n = surf[cur][?], surf?_o = surf[cur^1][?] (interior)
@@ -764,9 +765,11 @@ int record_step(cansfz_ctx* c, Recorder* rec, bool* complete, int levels) {
 // Levels per block of the tile kernels in an ensemble's step.  32 levels spend
 // 6% on the planes a block loads beyond its own (8 levels: 25%), which is what
 // counts when the cases fill the GPU; with less work their latency does, one
-// level after the other.  Per pass of 8 steps with 32 -> 8 levels: 12 2-D and 12
-// 3-D cases (11.5 million cells) 20.9 -> 21.1 ms, 12 2-D ones (1.1 million) 6.1 ->
-// 5.6 ms, 4 and 4 (4 million) 5.3 -> 4.6 ms.
+// level after the other.  Per 8 steps with 32 -> 8 levels, 2-D + 3-D cases:
+// 4+4 (1.4 million cells) 3.70 -> 2.95 ms, 12+0 (1.2) 3.68 -> 3.19, 6+6 (2.2)
+// 4.58 -> 4.20; from 4 to 8 million cells no difference beyond 1% either way
+// (7+7, 8+8, 9+9, 10+10, 0+6, 0+8, 12+6); 12+12 (9.7) 14.91 -> 15.00.  The line
+// is the upper end of that flat range.
 int ensemble_levels(const std::vector<cansfz_ctx*>& cases) {
   double cells = 0.;
   for (const cansfz_ctx* c : cases) cells += (double)c->g.tsize();

@@ -229,9 +229,10 @@ void launch_bc_group(const Launch& L, const Geo& g, const BcGroup& grp, const De
         planes[d] = face ? 3 : (planes[d] > 2 ? planes[d] : 2);
       }
     if (one) {
-      const long long n = (long long)planes[2] * NX * NY + (long long)planes[1] * NX * NZ + (long long)planes[0] * NY * NZ;
+      const long long n =
+          (long long)planes[2] * NX * NY + (long long)planes[1] * NX * NZ + (long long)planes[0] * NY * NZ;
       kgo_chain<BcAll, 256, 1>(L, k_bc_all, dim3((unsigned)((n + tb - 1) / tb), grp.nf), tb, 0, g, grp, sc, planes[0],
-                         planes[1], planes[2]);
+                               planes[1], planes[2]);
       return;
     }
   }
@@ -239,9 +240,10 @@ void launch_bc_group(const Launch& L, const Geo& g, const BcGroup& grp, const De
     const int n = 2 * NX * NZ + 2 * NX * NY;
     kgo_chain<BcStage<ST_PER>, 256, 1>(L, k_bc_stage<ST_PER>, dim3((n + tb - 1) / tb, grp.nf), tb, 0, g, grp, sc);
   }
-  if (any_x) kgo_chain<BcStage<ST_X>, 256, 1>(L, k_bc_stage<ST_X>, dim3((NY * NZ + tb - 1) / tb, grp.nf), tb, 0, g, grp, sc);
-  if (any_y) kgo_chain<BcStage<ST_Y>, 256, 1>(L, k_bc_stage<ST_Y>, dim3((NX * NZ + tb - 1) / tb, grp.nf), tb, 0, g, grp, sc);
-  if (any_z) kgo_chain<BcStage<ST_Z>, 256, 1>(L, k_bc_stage<ST_Z>, dim3((NX * NY + tb - 1) / tb, grp.nf), tb, 0, g, grp, sc);
+  auto plane = [&](int n) { return dim3((n + tb - 1) / tb, grp.nf); };
+  if (any_x) kgo_chain<BcStage<ST_X>, 256, 1>(L, k_bc_stage<ST_X>, plane(NY * NZ), tb, 0, g, grp, sc);
+  if (any_y) kgo_chain<BcStage<ST_Y>, 256, 1>(L, k_bc_stage<ST_Y>, plane(NX * NZ), tb, 0, g, grp, sc);
+  if (any_z) kgo_chain<BcStage<ST_Z>, 256, 1>(L, k_bc_stage<ST_Z>, plane(NX * NY), tb, 0, g, grp, sc);
 }
 
 // updt_rhs_b, src/bound.f90:341-396 (c_or_f = 'c', so q = 0): add the BC

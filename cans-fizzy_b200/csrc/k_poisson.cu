@@ -1624,7 +1624,8 @@ __global__ void __launch_bounds__(128) k_zsolve(int ncol, int nz, const double* 
 // 3P to CH*P); EXACT: every chunk has CH levels.  What bounds it depends on
 // the grid: with many columns the FP64 reciprocals and the shared memory (two
 // blocks per SM at nz = 256), with few the length of the chain of dependent
-// steps, CH + 2P + 2P + 2CH against the column sweep's 2 nz (a whole step at 64x64x128: 203 -> 184 us, at 64x2x128: 138 -> 126 us, the solve itself 28 -> 9 us).
+// steps, CH + 2P + 2P + 2CH against the column sweep's 2 nz (a whole step at
+// 64x64x128: 203 -> 184 us, at 64x2x128: 138 -> 126 us, the solve itself 28 -> 9 us).
 //
 // Pivots without cancellation.  b + lambda - a*d, gaussel's pivot
 // (src/solver.f90:151-177), is the difference of nearly equal numbers where
@@ -1737,7 +1738,8 @@ struct ZSolvePart {
     T* xb = red + (size_t)8 * P * NC;              // [2P][NC]: x_s, x_e of every chunk
     T* sum = xb + (size_t)2 * P * NC;              // [nz]: the rows' sums a + b + c
     const bool serial0 = zsing && __ldg(lam) == 0.;
-    if (zsing && bk.x == 0) {  // the extra block, first: its chain is the longest (as the last one: 94 -> 101 us at 256^3)
+    // the extra block, first: its chain is the longest (as the last one: 94 -> 101 us at 256^3)
+    if (zsing && bk.x == 0) {
       if (serial0) zsolve_serial0<T>(ncol, nz, a, b, c, piv0, df0, work, zsing, tile);
       return;
     }
@@ -2079,11 +2081,11 @@ static void x_forward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl,
       using X = FftX2Fwd<T, true, MC>;
       const dim3 g2((nlines + X::L - 1) / X::L);
       if (fused)
-        kgo_chain<FftX2Fwd<T, true, MC>, X::NT, 3>(Lc, k_fft_x2_fwd<T, true, MC>, g2, X::NT, 0, g, pl.px, sc, nullptr, u, v,
-                                            w, *ph, wbuf<T>(pl));
+        kgo_chain<FftX2Fwd<T, true, MC>, X::NT, 3>(Lc, k_fft_x2_fwd<T, true, MC>, g2, X::NT, 0, g, pl.px, sc, nullptr,
+            u, v, w, *ph, wbuf<T>(pl));
       else
         kgo_chain<FftX2Fwd<T, false, MC>, X::NT, 3>(Lc, k_fft_x2_fwd<T, false, MC>, g2, X::NT, 0, g, pl.px, sc, src,
-                                             nullptr, nullptr, nullptr, pz, wbuf<T>(pl));
+            nullptr, nullptr, nullptr, pz, wbuf<T>(pl));
       return;
     }
   }
@@ -2091,11 +2093,11 @@ static void x_forward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl,
     if (pl.px.kind == 0 && pl.lmode == 0) {
       const dim3 g5((nlines + kW - 1) / kW);
       if (fused)
-        kgo_chain<FftXWFwd<T, true>, 256, 2>(Lc, k_fft_x512_fwd<T, true>, g5, 256, w512_smem<T>(true), g, pl.px, sc, nullptr,
-                                       u, v, w, *ph, wbuf<T>(pl));
+        kgo_chain<FftXWFwd<T, true>, 256, 2>(Lc, k_fft_x512_fwd<T, true>, g5, 256, w512_smem<T>(true), g, pl.px, sc,
+            nullptr, u, v, w, *ph, wbuf<T>(pl));
       else
-        kgo_chain<FftXWFwd<T, false>, 256, 2>(Lc, k_fft_x512_fwd<T, false>, g5, 256, w512_smem<T>(true), g, pl.px, sc, src,
-                                        nullptr, nullptr, nullptr, pz, wbuf<T>(pl));
+        kgo_chain<FftXWFwd<T, false>, 256, 2>(Lc, k_fft_x512_fwd<T, false>, g5, 256, w512_smem<T>(true), g, pl.px, sc,
+            src, nullptr, nullptr, nullptr, pz, wbuf<T>(pl));
       return;
     }
   }
@@ -2104,20 +2106,20 @@ static void x_forward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl,
       constexpr int R = MC / 32;
       const dim3 gw((nlines + 8 * kWarpLines - 1) / (8 * kWarpLines));
       if (fused)
-        kgo_chain<FftXFwdW<T, true, R>, 256, 1>(Lc, k_fft_x_fwd_w<T, true, R>, gw, 256, 0, g, pl.px, sc, nullptr, u, v, w,
-                                          *ph, wbuf<T>(pl));
+        kgo_chain<FftXFwdW<T, true, R>, 256, 1>(Lc, k_fft_x_fwd_w<T, true, R>, gw, 256, 0, g, pl.px, sc, nullptr, u, v,
+            w, *ph, wbuf<T>(pl));
       else
         kgo_chain<FftXFwdW<T, false, R>, 256, 1>(Lc, k_fft_x_fwd_w<T, false, R>, gw, 256, 0, g, pl.px, sc, src, nullptr,
-                                           nullptr, nullptr, pz, wbuf<T>(pl));
+            nullptr, nullptr, pz, wbuf<T>(pl));
       return;
     }
   }
   if (fused)
     kgo_chain<FftXFwd<T, true, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_fwd<T, true, MC, xL<T, MC>()>, grid, 256, smem, g,
-                                                   pl.px, sc, nullptr, u, v, w, *ph, wbuf<T>(pl), L);
+        pl.px, sc, nullptr, u, v, w, *ph, wbuf<T>(pl), L);
   else
-    kgo_chain<FftXFwd<T, false, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_fwd<T, false, MC, xL<T, MC>()>, grid, 256, smem, g,
-                                                    pl.px, sc, src, nullptr, nullptr, nullptr, pz, wbuf<T>(pl), L);
+    kgo_chain<FftXFwd<T, false, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_fwd<T, false, MC, xL<T, MC>()>, grid, 256, smem,
+        g, pl.px, sc, src, nullptr, nullptr, nullptr, pz, wbuf<T>(pl), L);
 }
 
 template <typename T>
@@ -2161,10 +2163,10 @@ static void y_pass_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl, co
   const dim3 grid((g.nx + L - 1) / L, g.nz);
   if (dir > 0)
     kgo_chain<FftY<T, 1, MC, yL<T, MC>()>, 256, 1>(Lc, k_fft_y<T, 1, MC, yL<T, MC>()>, grid, 256, smem, g, pl.py, sc,
-                                             wbuf<T>(pl), L);
+        wbuf<T>(pl), L);
   else
     kgo_chain<FftY<T, -1, MC, yL<T, MC>()>, 256, 1>(Lc, k_fft_y<T, -1, MC, yL<T, MC>()>, grid, 256, smem, g, pl.py, sc,
-                                              wbuf<T>(pl), L);
+        wbuf<T>(pl), L);
 }
 
 template <typename T>
@@ -2207,9 +2209,8 @@ static void z_part_go(const Launch& Lc, const Geo& g, const PoissonPlan& pl, con
   constexpr int MINB = P == 8 ? (sizeof(T) == 4 ? 4 : 2) : 1;
   // the tiles of columns, and before them the block of the singular column
   kgo_chain<ZSolvePart<T, CH, P, EXACT>, 32 * P, MINB>(Lc, k_zsolve_part<T, CH, P, EXACT>,
-                                                 (ncol + ZP_NC - 1) / ZP_NC + (pl.zsing ? 1 : 0),
-                                                 32 * P, zpart_smem<T>(g.nz, P), ncol, g.nz, pl.lam, pl.a, pl.b, pl.c,
-                                                 zpiv0<T>(pl), zdf0<T>(pl), sc, wbuf<T>(pl), pl.zsing);
+      (ncol + ZP_NC - 1) / ZP_NC + (pl.zsing ? 1 : 0), 32 * P, zpart_smem<T>(g.nz, P), ncol, g.nz, pl.lam, pl.a, pl.b,
+      pl.c, zpiv0<T>(pl), zdf0<T>(pl), sc, wbuf<T>(pl), pl.zsing);
 }
 template <typename T, int CH, int P>
 static void z_part_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl, const DevScalars* sc) {
@@ -2249,20 +2250,20 @@ static void z_pass(const Launch& Lc, const Geo& g, const PoissonPlan& pl, const 
   if (zpiv<T>(pl) && zdf<T>(pl)) {
     if (pl.zper)
       kgo_chain<ZSolvePeriodicF<T>, 128, 1>(Lc, k_zsolve_periodic_f<T>, (ncol + tb - 1) / tb, tb, 0, ncol, g.nz, pl.lam,
-                                      pl.a, pl.b, pl.c, zpiv<T>(pl), zdf<T>(pl), sc, wbuf<T>(pl), wbuf2<T>(pl));
+          pl.a, pl.b, pl.c, zpiv<T>(pl), zdf<T>(pl), sc, wbuf<T>(pl), wbuf2<T>(pl));
     else
       kgo_chain<ZSolveF<T>, 128, 1>(Lc, k_zsolve_f<T>, (ncol + tb - 1) / tb, tb, 0, ncol, g.nz, pl.a, zpiv<T>(pl),
-                              zdf<T>(pl), sc, wbuf<T>(pl));
+          zdf<T>(pl), sc, wbuf<T>(pl));
     return;
   }
   const int nch = (g.nz + ZCH - 1) / ZCH;
   const size_t smem = (size_t)nch * tb * sizeof(T);
   if (pl.zper)
     kgo_chain<ZSolvePeriodic<T>, 128, 1>(Lc, k_zsolve_periodic<T>, (ncol + tb - 1) / tb, tb, smem, ncol, g.nz, pl.lam,
-                                   pl.a, pl.b, pl.c, sc, wbuf<T>(pl), wbuf2<T>(pl));
+        pl.a, pl.b, pl.c, sc, wbuf<T>(pl), wbuf2<T>(pl));
   else
     kgo_chain<ZSolve<T>, 128, 1>(Lc, k_zsolve<T>, (ncol + tb - 1) / tb, tb, smem, ncol, g.nz, pl.lam, pl.a, pl.b, pl.c,
-                           sc, wbuf<T>(pl), pl.zsing);
+        sc, wbuf<T>(pl), pl.zsing);
 }
 
 template <typename T, bool ADD, int MC>
@@ -2276,28 +2277,28 @@ static void x_backward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl
     if (pl.px.kind == 0 && pl.lmode == 0) {
       using X = FftX2Bwd<T, ADD, MC>;
       kgo_chain<FftX2Bwd<T, ADD, MC>, X::NT, 4>(Lc, k_fft_x2_bwd<T, ADD, MC>, (nlines + X::L - 1) / X::L, X::NT, 0, g,
-                                         pl.px, sc, wbuf<T>(pl), pl.normfft, dst, ADD ? 0 : Lc.wrap);
+          pl.px, sc, wbuf<T>(pl), pl.normfft, dst, ADD ? 0 : Lc.wrap);
       return;
     }
   }
   if constexpr (MC == 256) {
     if (pl.px.kind == 0 && pl.lmode == 0) {
-      kgo_chain<FftXWBwd<T, ADD>, 256, 2>(Lc, k_fft_x512_bwd<T, ADD>, (nlines + kW - 1) / kW, 256, w512_smem<T>(true), g,
-                                    pl.px, sc, wbuf<T>(pl), pl.normfft, dst, ADD ? 0 : Lc.wrap);
+      kgo_chain<FftXWBwd<T, ADD>, 256, 2>(Lc, k_fft_x512_bwd<T, ADD>, (nlines + kW - 1) / kW, 256, w512_smem<T>(true),
+          g, pl.px, sc, wbuf<T>(pl), pl.normfft, dst, ADD ? 0 : Lc.wrap);
       return;
     }
   }
   if constexpr (MC == 64 || MC == 128) {
     if (pl.px.kind == 0) {
       constexpr int R = MC / 32;
-      kgo_chain<FftXBwdW<T, ADD, R>, 256, 1>(Lc, k_fft_x_bwd_w<T, ADD, R>, (nlines + 8 * kWarpLines - 1) / (8 * kWarpLines),
-                                       256, 0, g, pl.px, sc, wbuf<T>(pl), pl.normfft, dst, ADD ? 0 : Lc.wrap);
+      kgo_chain<FftXBwdW<T, ADD, R>, 256, 1>(Lc, k_fft_x_bwd_w<T, ADD, R>,
+          (nlines + 8 * kWarpLines - 1) / (8 * kWarpLines), 256, 0, g, pl.px, sc, wbuf<T>(pl), pl.normfft, dst,
+          ADD ? 0 : Lc.wrap);
       return;
     }
   }
-  kgo_chain<FftXBwd<T, ADD, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_bwd<T, ADD, MC, xL<T, MC>()>, (nlines + L - 1) / L, 256,
-                                                smem, g, pl.px, sc, wbuf<T>(pl), pl.normfft, dst, L,
-                                                ADD ? 0 : Lc.wrap);
+  kgo_chain<FftXBwd<T, ADD, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_bwd<T, ADD, MC, xL<T, MC>()>, (nlines + L - 1) / L,
+      256, smem, g, pl.px, sc, wbuf<T>(pl), pl.normfft, dst, L, ADD ? 0 : Lc.wrap);
 }
 
 template <typename T, bool ADD>

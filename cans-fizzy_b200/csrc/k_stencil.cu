@@ -234,11 +234,11 @@ void launch_cmpt_phi_f32(const Launch& L, const Geo& g, const DevScalars* sc, bo
   const int n = g.hsize();
   if (narrow_only) kgo<Narrow, 256, 1>(L, k_narrow, (n + 255) / 256, 256, 0, n, sc, psi, phi);
   else if (acdi)
-    kgo_chain<CmptPhi<true, float>, 256, 1>(L, k_cmpt_phi<true, float>, (n + 256 * kPhiPer - 1) / (256 * kPhiPer), 256, 0,
-                                      n, sc, psi, phi);
+    kgo_chain<CmptPhi<true, float>, 256, 1>(L, k_cmpt_phi<true, float>, (n + 256 * kPhiPer - 1) / (256 * kPhiPer), 256,
+        0, n, sc, psi, phi);
   else
-    kgo_chain<CmptPhi<false, float>, 256, 1>(L, k_cmpt_phi<false, float>, (n + 256 * kPhiPer - 1) / (256 * kPhiPer), 256,
-                                       0, n, sc, psi, phi);
+    kgo_chain<CmptPhi<false, float>, 256, 1>(L, k_cmpt_phi<false, float>, (n + 256 * kPhiPer - 1) / (256 * kPhiPer),
+        256, 0, n, sc, psi, phi);
 }
 
 // ---------------------------------------------------------------------------

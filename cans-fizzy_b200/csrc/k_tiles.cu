@@ -199,7 +199,8 @@ struct YoungsTile {
   }
 };
 template <typename TI, int TYV>
-__global__ void __launch_bounds__(tile::Shape<TYV>::NT + tile::Shape<TYV>::TX, 4) k_youngs_tile(Geo g, const DevScalars* sc, int kz,
+__global__ void __launch_bounds__(tile::Shape<TYV>::NT + tile::Shape<TYV>::TX, 4) k_youngs_tile(Geo g,
+                                                          const DevScalars* sc, int kz,
                                                           const TI* phi, TI* __restrict__ normx,
                                                           TI* __restrict__ normy, TI* __restrict__ normz,
                                                           TI* __restrict__ kappa, int wrap) {
@@ -416,7 +417,8 @@ struct AcdiTile {
 template <typename TI>
 constexpr int acdi_blocks() { return sizeof(TI) == 8 ? 3 : 4; }
 template <typename TI, bool SDF, bool UPD, int TYV>
-__global__ void __launch_bounds__(tile::Shape<TYV>::TX * (tile::Shape<TYV>::TY + 1), acdi_blocks<TI>()) k_acdi_tile(Geo g, const DevScalars* sc, int kz,
+__global__ void __launch_bounds__(tile::Shape<TYV>::TX * (tile::Shape<TYV>::TY + 1), acdi_blocks<TI>())
+k_acdi_tile(Geo g, const DevScalars* sc, int kz,
     const double* u, const double* v, const double* w,
     const TI* nx_, const TI* ny_, const TI* nz_,
     const TI* phi, const double* psi, TI* __restrict__ dpsidt,
@@ -434,7 +436,7 @@ static void youngs_go(const Launch& L, const Geo& g, const DevScalars* sc, const
   using S = tile::Shape<TYV>;
   const int kz = tile::kz_of<TYV>(g, L.batched, L.nsm, L.phase_slots > 0 ? L.phase_slots : 24, TYV == 8 ? 4 : 8);
   kgo_chain<YoungsTile<TI, TYV>, S::NT + S::TX, 4>(L, k_youngs_tile<TI, TYV>, tile::grid_of<TYV>(g, kz),
-                                              dim3(S::TX, S::TY + 1), 0, g, sc, kz, phi, nx, ny, nz, kappa, L.wrap);
+      dim3(S::TX, S::TY + 1), 0, g, sc, kz, phi, nx, ny, nz, kappa, L.wrap);
 }
 
 template <typename TI>
@@ -451,9 +453,8 @@ static void acdi_go(const Launch& L, const Geo& g, const DevScalars* sc, const d
   using S = tile::Shape<TYV>;
   const int kz = tile::kz_of<TYV>(g, L.batched, L.nsm, L.phase_slots > 0 ? L.phase_slots : 24, TYV == 8 ? 3 : 6);
   kgo_chain<AcdiTile<TI, SDF, UPD, TYV>, S::TX * (S::TY + 1), acdi_blocks<TI>()>(L, k_acdi_tile<TI, SDF, UPD, TYV>,
-                                             tile::grid_of<TYV>(g, kz),
-                                             dim3(S::TX, S::TY + 1), acdi_smem<TI, SDF, TYV>(), g, sc, kz, u, v, w, nx,
-                                             ny, nz, phi, psi, hist, fx, fy, fz, psi_out, L.wrap);
+      tile::grid_of<TYV>(g, kz), dim3(S::TX, S::TY + 1), acdi_smem<TI, SDF, TYV>(), g, sc, kz, u, v, w, nx, ny, nz, phi,
+      psi, hist, fx, fy, fz, psi_out, L.wrap);
 }
 
 template <typename TI, int TYV>

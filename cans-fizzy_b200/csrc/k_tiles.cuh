@@ -51,9 +51,9 @@ __device__ __forceinline__ bool plane_cell(const Geo& g, int i0, int j0, int kk,
 // The elements of a plane that one of NTH threads copies, placed once instead of
 // at every level: element q at halo index off + kk*sxy, or nothing (a zero)
 // outside the array.  With the ring slots rotated instead of reduced modulo 3, at
-// 256^3: ACDI tile 527 -> 516 us (FP32 383 -> 371), Youngs 272 -> 247 us (FP32 220
-// -> 192): both issue about 70% of the slots, over a third of them integer
-// arithmetic.
+// 256^3: ACDI tile 527 -> 516 us (FP32 383 -> 371, a fourth block per SM
+// included), Youngs 272 -> 247 us (FP32 220 -> 192): both issue about 70% of the
+// slots, over a third of them integer arithmetic.
 template <int PX, int PXY, int NTH>
 struct PlaneCopy {
   static constexpr int NE = (PXY + NTH - 1) / NTH;

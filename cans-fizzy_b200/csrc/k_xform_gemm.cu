@@ -319,7 +319,8 @@ __global__ void __launch_bounds__(GTHREADS, 2) k_xform_gemm(GemmXform p, DevScal
       } else {
 #pragma unroll
         for (int i = 0; i < 16; ++i)
-          split_store2(ahi, alo, apair + (uint32_t)(i >> 3) * GSBO + (uint32_t)(i & 7) * 16, x.v[2 * i], x.v[2 * i + 1]);
+          split_store2(ahi, alo, apair + (uint32_t)(i >> 3) * GSBO + (uint32_t)(i & 7) * 16, x.v[2 * i],
+                       x.v[2 * i + 1]);
       }
       fence_async_smem();
       __syncthreads();

@@ -93,8 +93,9 @@ typedef struct cansfz_params {
                                    FP32 Poisson solve; -1: the Poisson solve in FP64 */
   int32_t fp32_transforms;      /* mixed form, FP32 solve: 0 = x/y line transforms as
                                    split-BF16 GEMMs on the tensor cores (tcgen05) where
-                                   the line lengths are 64, 128 or 256, shared-memory FFTs
-                                   otherwise; 1 = shared-memory FFTs always          */
+                                   the line lengths are 64, 128 or 256, FFTs otherwise;
+                                   1 = FFTs always (register passes for periodic lines
+                                   of 64 to 512 = 2^n points, else in shared memory)  */
   int32_t reserved[7];
 } cansfz_params;
 
@@ -315,7 +316,13 @@ int cansfz_profile_stages(cansfz_ctx* ctx, int nsteps, double* ms, int maxstages
  * FP32 spectral solve of the same discrete operator as cansfz_solver, then
  * `sweeps` refinement sweeps p += S32(rhs - L(p)) with the FP64 residual of
  * the 7-point Laplacian.  rhs and p: halo-layout device fields (p's ghost
- * layer is filled on return).  Homogeneous pressure BCs only.             */
+ * layer is filled on return).  Homogeneous pressure BCs only.
+ * Without a Dirichlet wall the system is singular: a solution exists where
+ * the dz-weighted mean of rhs is zero, as that of fillps is, and p is then
+ * defined up to a constant.  For another rhs the two solvers return results
+ * that differ, beyond the constant, in proportion to that mean, whatever the
+ * sweeps (1.4e-6 of the solution at 20x6x31, where the z quotients' single
+ * precision leaves dz uneven by 2e-6 and rhs has a plain mean of zero).    */
 int cansfz_solver_refined(cansfz_ctx* ctx, const double* rhs, double* p, int sweeps);
 /* FP64 residual res = rhs - L(p) of that operator (p's ghosts are filled). */
 int cansfz_poisson_residual(cansfz_ctx* ctx, const double* rhs, double* p, double* res);
