@@ -2018,9 +2018,13 @@ template <typename T, int CH, int P, bool EXACT>
 static void set_attr_zpart() {
   cudaFuncSetAttribute(k_zsolve_part<T, CH, P, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)zpart_smem<T>(CH * P, P));
-  // all of the unified L1/shared storage as shared memory: 2 FP64 or 4 FP32
-  // tiles per SM at 256 levels
-  cudaFuncSetAttribute(k_zsolve_part<T, CH, P, EXACT>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  // No preference for the split of L1 and shared memory: the driver's makes room
+  // for the two FP64 or four FP32 tiles per SM at 256 levels by itself.  A
+  // preference for all of it as shared memory, unlike the other kernels', left
+  // the kernel as fast (92 us at 256^3) or up to 2 us slower, and made SMs drain to
+  // change the split when several cases' kernels are on the device: of three cases
+  // in turn, fillps + solve + fill took 437 us at 256^3 with it and 407 without,
+  // 135 and 121 at 128x128x256, 108 and 95 at 128x128x200.
 }
 template <typename T>
 static void set_attrs_zpart() {
