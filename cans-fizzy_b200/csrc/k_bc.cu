@@ -188,16 +188,6 @@ __global__ void k_bc_all(Geo g, BcGroup grp, const DevScalars* sc, int px, int p
   BcAll::run(blk_chain(), g, grp, sc, px, py, pz);
 }
 
-// Beyond this many points (48 MB; three such fields are more than the L2 holds)
-// a fill keeps its stages.  One launch is 4 to 6 us shorter than three at any
-// size, which is 1% of fillps + solve + fill of one case at 256^3 (441 -> 436
-// us).  But when a program has several cases in flight on streams of their own,
-// the short launches are what holds one case back while another's solve runs
-// through on fields still in L2: of three cases in turn a pass took 276 us with
-// stages and 284 with one launch at 192^3, 468 and 479 at 256^3, 1444 and 1543
-// at 320x256x256; at 160^3 479 and 475, at 128^3 65 and 58, at 64^3 27 and 22.
-constexpr int kFillOneLaunch = 6000000;
-
 void launch_bc_group(const Launch& L, const Geo& g, const BcGroup& grp, const DevScalars* sc) {
   if (grp.nf <= 0) return;
   bool any_per = false, any_x = false, any_y = false, any_z = false;
@@ -211,9 +201,8 @@ void launch_bc_group(const Launch& L, const Geo& g, const BcGroup& grp, const De
   const int NX = g.nx + 2, NY = g.ny + 2, NZ = g.nz + 2;
   const int tb = 256;
   // two or more stages: one launch (the 27 fills of a pass of procedures at
-  // 48x40x56: 195 -> 74 us, at 128^3: 235 -> 112 us), for fields of up to
-  // kFillOneLaunch points
-  if ((int)any_per + any_x + any_y + any_z >= 2 && g.hsize() <= kFillOneLaunch) {
+  // 48x40x56: 195 -> 74 us, at 128^3: 235 -> 112 us)
+  if ((int)any_per + any_x + any_y + any_z >= 2) {
     int planes[3] = {0, 0, 0};
     bool one = true;
     for (int f = 0; f < grp.nf; ++f)

@@ -82,17 +82,6 @@ def test_rk_2fl_in_one_pass(ng, vof):
 @pytest.mark.parametrize("cbcpre", ["PPPPNN", "NNPPNN", "DDPPNN", "PPNNNN", "PPPPPP", "NNNNNN", "DDNNDD", "PPPPDD"])
 @pytest.mark.parametrize("ng", [(24, 16, 20), (6, 2, 3), (36, 6, 9)])
 def test_ghost_fills_in_one_launch(cbcpre, ng):
-    _ghost_fills(cbcpre, ng)
-
-
-@pytest.mark.parametrize("cbcpre", ["PPPPNN", "NNPPNN", "DDNNDD"])
-@pytest.mark.parametrize("ng", [(200, 160, 180), (210, 168, 170)])
-def test_ghost_fills_beside_the_line_between_one_launch_and_stages(cbcpre, ng):
-    assert ((ng[0] + 2) * (ng[1] + 2) * (ng[2] + 2) <= 6000000) == (ng[0] == 200)
-    _ghost_fills(cbcpre, ng)
-
-
-def _ghost_fills(cbcpre, ng):
     p = _nml(*ng, cbcpre, l=(1.0, 0.75, 1.2))
     for q in range(18):
         p.bcvel[q] = 0.1 * q - 0.3
