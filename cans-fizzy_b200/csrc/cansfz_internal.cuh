@@ -198,8 +198,8 @@ struct PoissonPlan {
   // split-BF16 matrices [0] forward, [1] backward; null: the FFT kernels
   const uint16_t* gx[2];
   const uint16_t* gy[2];
-  // z solve: 0 the partitioned tile solve where it applies, 1 one column per
-  // thread (cansfz_plan.zsolve)
+  // z solve: 0 the partitioned tile solve where it applies and is the faster
+  // one, 1 one column per thread (cansfz_plan.zsolve)
   int zmode;
   // x and y transforms of the periodic kind: 0 the two-pass register
   // kernels where the length allows, 1 the one-warp-per-line (x) and
@@ -378,7 +378,12 @@ void poisson_set_attributes();
 double xform_coef(int kind, int dir, int n, int j, int k);
 std::vector<uint16_t> xform_bmat(int kind, int dir, int n);
 bool xform_gemm_length(int n);
+// the partitioned z solve can take the grid's columns, and (in FP64 or FP32) it
+// does under the plan
 bool z_part_ok(const Geo& g, const PoissonPlan& pl);
+bool z_part_takes(const Geo& g, const PoissonPlan& pl, bool f32);
+// column solves of fewer columns than this read precomputed elimination factors
+constexpr int kZFactored = 32768;
 // the x or y transforms have a two-pass register kernel (periodic kind, 64-512 points)
 bool poisson_y2_applies(const PoissonPlan& pl);
 int xform_gemm_set_attributes();

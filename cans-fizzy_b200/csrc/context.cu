@@ -306,17 +306,17 @@ bool factorize(int m, int radix[FFT_MAXSTAGES], int* nst) {
 // evaluates its own, does not take the columns.
 int alloc_z_factors(cansfz_ctx* c) {
   PoissonPlan& pl = c->pl;
-  if ((long long)c->g.nx * c->g.ny >= 32768 || (pl.zmode != 1 && z_part_ok(c->g, pl))) return CANSFZ_OK;
-  const size_t nint = (size_t)c->g.tsize();
   const int ncol = c->g.nx * c->g.ny;
+  if (ncol >= kZFactored) return CANSFZ_OK;
+  const size_t nint = (size_t)c->g.tsize();
   int rc;
-  if (!pl.zdf) {
+  if (!pl.zdf && !z_part_takes(c->g, pl, false)) {
     if (!pl.zpiv && (rc = dalloc(c, &pl.zpiv, nint))) return rc;
     if ((rc = dalloc(c, &pl.zdf, nint))) return rc;
     launch_z_factors(c->L, c->g, pl, false, ncol, pl.zpiv, pl.zdf);
     CK(cudaGetLastError());
   }
-  if (pl.workf && !pl.zdff) {
+  if (pl.workf && !pl.zdff && !z_part_takes(c->g, pl, true)) {
     if (!pl.zpivf && (rc = dalloc(c, &pl.zpivf, nint))) return rc;
     if ((rc = dalloc(c, &pl.zdff, nint))) return rc;
     launch_z_factors(c->L, c->g, pl, true, ncol, pl.zpivf, pl.zdff);

@@ -2232,12 +2232,30 @@ bool poisson_y2_applies(const PoissonPlan& pl) {
 bool z_part_ok(const Geo& g, const PoissonPlan& pl) {
   return !pl.zper && (g.nx * g.ny) % 4 == 0 && zpart_chunks(g.nz) != 0;
 }
+// ... and it does where it is the faster one.  It takes two reciprocals per
+// level and a reduced system per column; a column solve one (or, below 32768
+// columns, reads its factors) and a chain of 2 nz steps.  Short columns of a grid
+// that fills the device with them are the column solve's.  The z solve alone,
+// column against partitioned, us:
+//   FP64  128x128x24   7.3/7.0   x40  9.8/8.3
+//         256x96x24    7.5/9.6   x48 11.4/12.5  x52 14.3/13.6  x64 16.0/13.6
+//         256x128x24  12.3/12.2  x36 18.5/14.4
+//         256x256x24  14.4/20.9  x36 21.0/25.2  x56 29.4/31.8  x64 32.0/30.8
+//         512x512x24  45.0/79.2  x56  107/125   x64  120/125
+//   FP32  256x96x24    7.7/7.5   512x256x24 26.2/24.8
+//         512x512x24  40.7/47.6  x32 48.3/53.2  x36 59.1/57.0  x64 92.4/72.1
+bool z_part_takes(const Geo& g, const PoissonPlan& pl, bool f32) {
+  if (pl.zmode == 1 || !z_part_ok(g, pl)) return false;
+  const int ncol = g.nx * g.ny, nz = g.nz;
+  if (f32) return nz >= 36 || ncol <= 131072;
+  return nz >= 64 || ncol <= 16384 || (ncol < kZFactored ? nz >= 52 : ncol <= 40000);
+}
 
 template <typename T>
 static void z_pass(const Launch& Lc, const Geo& g, const PoissonPlan& pl, const DevScalars* sc) {
   const int ncol = g.nx * g.ny;
   const int tb = 64;
-  if (pl.zmode != 1 && z_part_ok(g, pl)) {
+  if (z_part_takes(g, pl, sizeof(T) == 4)) {
     const int len = zpart_len(g.nz);
     if (zpart_chunks(g.nz) == 16) {
       if (len == 24) z_part_len<T, 24, 16>(Lc, g, pl, sc);

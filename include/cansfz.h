@@ -341,7 +341,8 @@ typedef struct cansfz_plan {
   int32_t momentum_slots;   /* the same for the momentum tile (default 48)   */
   int32_t zsolve;           /* Poisson z solve: 0 the partitioned 32-column
                                tiles where z is not periodic and has 24 to
-                               512 levels, 1 one column per thread            */
+                               512 levels (short columns of a grid of many:
+                               as 1), 1 one column per thread                 */
   int32_t fp32_transforms;  /* mixed form's FP32 solve: 0 tensor-core GEMMs
                                where the line lengths allow, 1 FFTs           */
   double  ms_per_step;      /* step time measured with the plan by
