@@ -754,7 +754,7 @@ void launch_fillps(const Launch& L, const Geo& g, const Phys& ph, const DevScala
 __global__ void k_correc(Geo g, Phys ph, const DevScalars* __restrict__ sc, const double* __restrict__ p,
                          double* __restrict__ u, double* __restrict__ v, double* __restrict__ w) {
   if (HALTED(sc)) return;
-  const int i = blockIdx.x * 32 + threadIdx.x, j = blockIdx.y * 8 + threadIdx.y, k = blockIdx.z;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y, k = blockIdx.z;
   if (i > g.nx + 1 || j > g.ny + 1) return;
   const double dt = sc->dt, rhop = ph.rho0;
   const int c = g.h(i, j, k);
@@ -765,9 +765,16 @@ __global__ void k_correc(Geo g, Phys ph, const DevScalars* __restrict__ sc, cons
 }
 void launch_correc(const Launch& L, const Geo& g, const Phys& ph, const DevScalars* sc, const double* p, double* u,
                    double* v, double* w) {
-  // 32x8 tiles: blocks of 128 along x left one of two nearly empty at nx = 128
-  // (34 -> 32 us)
-  const dim3 b(32, 8), gr((g.nx + 2 + 31) / 32, (g.ny + 2 + 7) / 8, g.nz + 2);
+  // Blocks of a row's 128 points (64 where it has fewer than 128), or tiles of
+  // 32x8 where those leave clearly fewer threads without a point: 128^3 (one of
+  // two row blocks nearly empty) 34 -> 32 us, 256^3 260 -> 257, 30x512x64 32 -> 22;
+  // but 1024x2x512, whose ny + 2 = 4 rows half fill a tile, 30 -> 38 us,
+  // 512x256x100, 15% fewer, 195 -> 200, and 384x384x128, 21% fewer, 281 -> 287.
+  const int X = g.nx + 2, Y = g.ny + 2, row = X >= 128 ? 128 : 64;
+  const long long rows = (long long)((X + row - 1) / row) * row * Y;
+  const long long tiles = (long long)((X + 31) / 32) * 32 * ((Y + 7) / 8) * 8;
+  const dim3 b = 1.22 * tiles < rows ? dim3(32, 8) : dim3(row, 1);
+  const dim3 gr((X + b.x - 1) / b.x, (Y + b.y - 1) / b.y, g.nz + 2);
   k_correc<<<gr, b, 0, L.st>>>(g, ph, sc, p, u, v, w);
 }
 

@@ -102,3 +102,18 @@ def test_ghost_fills_in_one_launch(cbcpre, ng):
         o.call("bounduvw", correc, *uvw)
         for a, b in zip(dev, uvw):
             assert np.array_equal(a.get(), b), correc
+
+
+@pytest.mark.parametrize("ng", [(24, 16, 20), (126, 6, 9), (128, 14, 5), (10, 2, 9), (300, 2, 7), (6, 36, 3)])
+def test_correc_in_rows_and_in_tiles(ng):
+    """correc's two block shapes, ghost ranges included (its divisions by rho0
+    and the oracle's round alike: one rounding per operation)."""
+    p = _nml(*ng, "PPPPNN", l=(1.0, 0.75, 1.2))
+    g, o = C.Case(p), O.Case(p)
+    _, f, _ = _rand_fields(p, 41)
+    pp, u, v, w = (f() for _ in range(4))
+    dev = [g.field(a) for a in (u, v, w)]
+    g.call("correc", 0.013, g.field(pp), *dev)
+    o.call("correc", 0.013, pp, u, v, w)
+    for a, b in zip(dev, (u, v, w)):
+        assert _rel(a.get(), b) < 1e-14
