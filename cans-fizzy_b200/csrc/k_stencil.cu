@@ -264,9 +264,9 @@ struct PutFields {
   const double* src[3];
   double* dst[3];
 };
-// one warp per row, eight rows per block, field blockIdx.y; clip: the rows of
-// the ghost layer too
-__global__ void __launch_bounds__(256) k_put_interior(Geo g, PutFields f, int clip) {
+// one warp per row, eight rows per block, field blockIdx.y, points blockIdx.z*seg
+// to the next seg of each row; clip: the rows of the ghost layer too
+__global__ void __launch_bounds__(256) k_put_interior(Geo g, PutFields f, int clip, int seg) {
   const int lo = clip ? 0 : 1, ny = clip ? g.ny + 2 : g.ny, nz = clip ? g.nz + 2 : g.nz;
   const int r = blockIdx.x * 8 + threadIdx.y;
   if (r >= ny * nz) return;
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(256) k_put_interior(Geo g, PutFields f, int cl
   const bool row = j >= 1 && j <= g.ny && k >= 1 && k <= g.nz;
   const int c = g.h(0, j, k);
 #pragma unroll 4
-  for (int i = threadIdx.x + lo; i <= g.nx + 1 - lo; i += 32) {
+  for (int i = blockIdx.z * seg + threadIdx.x + lo; i < min((int)(blockIdx.z + 1) * seg + lo, g.nx + 2 - lo); i += 32) {
     if (row && i >= 1 && i <= g.nx) dst[c + i] = __ldg(src + c + i);
     else dst[c + i] = fmin(fmax(0., dst[c + i]), 1.);
   }
@@ -289,7 +289,11 @@ void launch_put_interior(const Launch& L, const Geo& g, int nf, const double* co
     f.dst[q] = dst[q];
   }
   const int rows = clip ? (g.ny + 2) * (g.nz + 2) : g.ny * g.nz;
-  k_put_interior<<<dim3((rows + 7) / 8, nf), dim3(32, 8), 0, L.st>>>(g, f, clip ? 1 : 0);
+  // long rows, but too few of them for four blocks per SM: split each
+  const int blocks = (rows + 7) / 8 * nf, want = 4 * (L.nsm > 0 ? L.nsm : 148);
+  const int n = clip ? g.nx + 2 : g.nx, parts = max(1, min((n + 127) / 128, want / blocks));
+  const int seg = ((n + parts - 1) / parts + 31) / 32 * 32;
+  k_put_interior<<<dim3((rows + 7) / 8, nf, (n + seg - 1) / seg), dim3(32, 8), 0, L.st>>>(g, f, clip ? 1 : 0, seg);
 }
 
 // ---------------------------------------------------------------------------

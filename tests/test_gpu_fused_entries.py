@@ -27,7 +27,7 @@ class _Shifted(C.DeviceField):
 
 @pytest.mark.parametrize("ng,opts,shifted", [((24, 16, 20), "", False), ((10, 2, 9), "", False), ((36, 10, 13), "", True),
                                              ((70, 6, 24), "balanced", False), ((24, 14, 9), "balanced", True),
-                                             ((24, 16, 20), "buoyancy", False)])
+                                             ((24, 16, 20), "buoyancy", False), ((300, 2, 9), "", False)])
 def test_rk_with_pn_equal_p(ng, opts, shifted):
     """rk called with pn = p, two calls (the history): the oracle, and the
     same call with a copy of p as pn, which takes the pass-by-pass route."""
@@ -60,7 +60,8 @@ def test_rk_with_pn_equal_p(ng, opts, shifted):
             assert np.array_equal(a.get()[ghosts], b.get()[ghosts])
 
 
-@pytest.mark.parametrize("ng,vof", [((36, 10, 13), False), ((10, 2, 9), False), ((36, 10, 13), True), ((64, 16, 24), True)])
+@pytest.mark.parametrize("ng,vof", [((36, 10, 13), False), ((10, 2, 9), False), ((36, 10, 13), True), ((64, 16, 24), True),
+                                    ((126, 2, 9), False), ((128, 2, 9), False), ((300, 4, 7), False), ((1024, 2, 5), True)])
 def test_rk_2fl_in_one_pass(ng, vof):
     p = _nml(*ng, "PPPPNN", l=(1.0, 0.75, 1.2), vof=vof)
     g, o = C.Case(p), O.Case(p)
