@@ -2002,6 +2002,18 @@ constexpr int yL() { return MC ? lines_per_cta(MC, y_maxL(MC), sizeof(T)) : 0; }
 // factors 2 and 3); other lengths take the runtime-length kernels
 #define CANSFZ_FOR_LENGTHS(X) X(16) X(24) X(32) X(48) X(64) X(96) X(128) X(192) X(256)
 
+// A Stockham pass over the lines of `p`: those of runtime length are long
+// kernels and, with at most a block per SM, not launched early (but for the
+// two-point lines of the 2-D convention, which are short).  A step at 30x200x30
+// 158 -> 141 us, 36x240x16 145 -> 137, 1000x2x100 with a refined solve 341 -> 263;
+// with 168 blocks (48x40x56) early is 2% faster.
+template <class F, int MC, class K, class... V>
+static void kgo_lines(const Launch& L, const LinePlan& p, K k, dim3 grid, int threads, size_t smem, V&&... v) {
+  const bool few = (long long)grid.x * grid.y * grid.z <= (L.nsm > 0 ? L.nsm : 148);
+  if (MC == 0 && p.m > 4 && few) kgo_spread<F, 256, 1>(L, k, grid, threads, smem, std::forward<V>(v)...);
+  else kgo_chain<F, 256, 1>(L, k, grid, threads, smem, std::forward<V>(v)...);
+}
+
 template <typename T, int MC>
 static void set_attr_len() {
   const int lim = 100 * 1024;
@@ -2119,11 +2131,11 @@ static void x_forward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl,
     }
   }
   if (fused)
-    kgo_chain<FftXFwd<T, true, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_fwd<T, true, MC, xL<T, MC>()>, grid, 256, smem, g,
-        pl.px, sc, nullptr, u, v, w, *ph, wbuf<T>(pl), L);
+    kgo_lines<FftXFwd<T, true, MC, xL<T, MC>()>, MC>(Lc, pl.px, k_fft_x_fwd<T, true, MC, xL<T, MC>()>, grid, 256, smem,
+        g, pl.px, sc, nullptr, u, v, w, *ph, wbuf<T>(pl), L);
   else
-    kgo_chain<FftXFwd<T, false, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_fwd<T, false, MC, xL<T, MC>()>, grid, 256, smem,
-        g, pl.px, sc, src, nullptr, nullptr, nullptr, pz, wbuf<T>(pl), L);
+    kgo_lines<FftXFwd<T, false, MC, xL<T, MC>()>, MC>(Lc, pl.px, k_fft_x_fwd<T, false, MC, xL<T, MC>()>, grid, 256,
+        smem, g, pl.px, sc, src, nullptr, nullptr, nullptr, pz, wbuf<T>(pl), L);
 }
 
 template <typename T>
@@ -2166,11 +2178,11 @@ static void y_pass_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl, co
   const size_t smem = 4 * (size_t)m * (L | 1) * sizeof(T);
   const dim3 grid((g.nx + L - 1) / L, g.nz);
   if (dir > 0)
-    kgo_chain<FftY<T, 1, MC, yL<T, MC>()>, 256, 1>(Lc, k_fft_y<T, 1, MC, yL<T, MC>()>, grid, 256, smem, g, pl.py, sc,
+    kgo_lines<FftY<T, 1, MC, yL<T, MC>()>, MC>(Lc, pl.py, k_fft_y<T, 1, MC, yL<T, MC>()>, grid, 256, smem, g, pl.py, sc,
         wbuf<T>(pl), L);
   else
-    kgo_chain<FftY<T, -1, MC, yL<T, MC>()>, 256, 1>(Lc, k_fft_y<T, -1, MC, yL<T, MC>()>, grid, 256, smem, g, pl.py, sc,
-        wbuf<T>(pl), L);
+    kgo_lines<FftY<T, -1, MC, yL<T, MC>()>, MC>(Lc, pl.py, k_fft_y<T, -1, MC, yL<T, MC>()>, grid, 256, smem, g, pl.py,
+        sc, wbuf<T>(pl), L);
 }
 
 template <typename T>
@@ -2319,7 +2331,7 @@ static void x_backward_len(const Launch& Lc, const Geo& g, const PoissonPlan& pl
       return;
     }
   }
-  kgo_chain<FftXBwd<T, ADD, MC, xL<T, MC>()>, 256, 1>(Lc, k_fft_x_bwd<T, ADD, MC, xL<T, MC>()>, (nlines + L - 1) / L,
+  kgo_lines<FftXBwd<T, ADD, MC, xL<T, MC>()>, MC>(Lc, pl.px, k_fft_x_bwd<T, ADD, MC, xL<T, MC>()>, (nlines + L - 1) / L,
       256, smem, g, pl.px, sc, wbuf<T>(pl), pl.normfft, dst, L, ADD ? 0 : Lc.wrap);
 }
 

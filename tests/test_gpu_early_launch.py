@@ -32,3 +32,10 @@ def test_many_steps_with_and_without_early_launch(ng, l, two_d, form):
     a, b = early.diag(), plain.diag()
     assert (a.istep, a.dt, a.gam, a.divmax) == (b.istep, b.dt, b.gam, b.divmax)
     ens.close()
+
+
+@pytest.mark.parametrize("ng", [(30, 200, 30), (250, 2, 40)])
+def test_lines_of_runtime_length_between_early_launches(ng):
+    """Transforms that are not launched early themselves, with kernels before
+    and after them that are."""
+    test_many_steps_with_and_without_early_launch(ng, (1.0, ng[1] / ng[0], ng[2] / ng[0]), ng[1] == 2, 0)
